@@ -26,6 +26,7 @@
 
 #include "check.cuh"
 #include "s3ttmc_chain.cuh"
+#include "s3ttmc_split.cuh"
 #include "s3ttmc_tiled.cuh"
 #include "s3ttmc_warp.cuh"
 #include "tensor.cuh"
@@ -440,6 +441,13 @@ uint32_t s3ttmc_launch_count(const TensorState &t, uint32_t R, bool packed) {
                      chain_supported(t, R);
   const uint32_t nsplit = chain && t.chain ? t.chain->nsplit : t.nsplit;
   uint32_t n = 1;                 // S3TTMc kernel
+  if (s3ttmc_schedule() == kScheduleAuto && split_supported(t.order, R)) {
+    ItemSet all;
+    all.nchunks = t.nchunks;
+    all.nheavy = t.nheavy;
+    const uint32_t nh = split_heavy(R, all);
+    if (nh && nh < t.nchunks) n += 1;  // warp kernel of the light rows
+  }
   if (chain && t.chain && t.chain->nlight) n += 1;  // warp kernel of the light rows
   if (nsplit) n += 1;             // combine kernel
   if (!packed) n += 1;            // unpack kernel
@@ -556,6 +564,32 @@ static void s3ttmc_items(TensorState &t, const ItemSet &items, const void *dU, u
     finish_rows(t, items, m, Ypk, packed, dY, R, L, precision, st);
     return;
   }
+  if (sched == kScheduleAuto && split_supported(t.order, R)) {
+    auto it = t.split_plans.find(R);
+    if (it == t.split_plans.end()) it = t.split_plans.emplace(R, split_plan(t.order, R)).first;
+    // small ranks: the light rows on the warp-per-row kernel (disjoint rows,
+    // on a side stream when there are rows of both kinds)
+    ItemSet heavy = items, light = items;
+    if (const uint32_t nh = split_heavy(R, items); nh < items.nchunks) {
+      heavy.nchunks = nh;
+      light.chunks += nh;
+      light.nchunks -= nh;
+      auto wt = t.warp.find(R);
+      if (wt == t.warp.end()) wt = t.warp.emplace(R, warp_plan(t.order, R)).first;
+      if (nh) {
+        SideFork fork(st);
+        warp_launch(*wt->second, t, light, dU, Ypk, precision, fork.side);
+        split_launch(*it->second, t, heavy, dU, Ypk, precision, st);
+        fork.join();
+      } else {
+        warp_launch(*wt->second, t, light, dU, Ypk, precision, st);
+      }
+    } else {
+      split_launch(*it->second, t, items, dU, Ypk, precision, st);
+    }
+    finish_rows(t, items, m, Ypk, packed, dY, R, L, precision, st);
+    return;
+  }
   if (sched == kScheduleAuto || sched == kScheduleWarp) {
     auto it = t.warp.find(R);
     if (it == t.warp.end()) it = t.warp.emplace(R, warp_plan(t.order, R)).first;
@@ -663,6 +697,7 @@ void s3ttmc_run(TensorState &t, const void *dU, uint32_t R, bool packed, void *d
   } else {
     all.chunks = t.chunks.p;
     all.nchunks = t.nchunks;
+    all.nheavy = t.nheavy;
     all.split = t.split.p;
     all.nsplit = t.nsplit;
     all.nslots = t.nslots;
@@ -757,6 +792,7 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
     band.rows = bd.row0[k + 1] - bd.row0[k];
     band.chain = chain;
     band.nslots = chain ? t.chain->nslots : t.nslots;
+    if (!chain) band.nheavy = bd.nheavy[k];
     if (chain) {
       band.light = bd.light.p + bd.light0[k];
       band.nlight = bd.light0[k + 1] - bd.light0[k];

@@ -172,6 +172,13 @@ void sort_heaviest_first(std::vector<Chunk> &ch, size_t b, size_t e, uint64_t ma
   std::copy(out.begin(), out.end(), ch.begin() + (std::ptrdiff_t)b);
 }
 
+// items of ch[b, e), heaviest first, with more than kLightOwners owners
+static uint32_t heavy_items(const std::vector<Chunk> &ch, size_t b, size_t e) {
+  size_t k = b;
+  while (k < e && ch[k].oe - ch[k].ob > kLightOwners) ++k;
+  return (uint32_t)(k - b);
+}
+
 void tensor_build(TensorState &t, const uint32_t *h_inds, const double *h_vals, bool on_device) {
   NvtxRange nv("tensor build");
   // SPB_TRACE_BUILD=1 prints the time of each phase (with a device sync)
@@ -299,8 +306,7 @@ void tensor_build(TensorState &t, const uint32_t *h_inds, const double *h_vals, 
   const uint32_t slot = row_order_items(t, ch, sp);
   sort_heaviest_first(ch, 0, ch.size(), co);
   t.nchunks = (uint32_t)ch.size();
-  t.nheavy = 0;
-  while (t.nheavy < t.nchunks && ch[t.nheavy].oe - ch[t.nheavy].ob > kLightOwners) ++t.nheavy;
+  t.nheavy = heavy_items(ch, 0, ch.size());
   t.nsplit = (uint32_t)sp.size();
   t.nslots = slot;
   t.chunks.alloc(ch.size());
@@ -343,7 +349,11 @@ const RowBands &row_bands(TensorState &t, uint32_t nb) {
                                                [](const SplitRow &c, uint32_t v) { return c.row < v; }) -
                               sp.begin());
   }
-  for (uint32_t k = 0; k < nb; ++k) sort_heaviest_first(ch, b->chunk0[k], b->chunk0[k + 1], t.chunk_owners);
+  b->nheavy.resize(nb);
+  for (uint32_t k = 0; k < nb; ++k) {
+    sort_heaviest_first(ch, b->chunk0[k], b->chunk0[k + 1], t.chunk_owners);
+    b->nheavy[k] = heavy_items(ch, b->chunk0[k], b->chunk0[k + 1]);
+  }
   b->chunks.alloc(ch.size());
   if (!ch.empty())
     SPB_CUDA(cudaMemcpy(b->chunks.p, ch.data(), ch.size() * sizeof(Chunk), cudaMemcpyHostToDevice));

@@ -36,9 +36,9 @@ struct Chunk {
   uint64_t ob, oe;
 };
 static constexpr uint32_t kDirect = 0xffffffffu;
-// work items with at most this many owners take one warp each in the
-// warp-per-owner S3TTMc schedule (larger ones take a whole CTA)
-static constexpr uint32_t kLightOwners = 48;
+// split-leaf schedule, R <= 8: work items with at most this many owners go to
+// the warp-per-row kernel (s3ttmc_split.cu)
+static constexpr uint32_t kLightOwners = 8;
 
 struct SplitRow {
   uint32_t row;
@@ -55,6 +55,7 @@ struct SplitRow {
 struct RowBands {
   uint32_t nb = 0;
   std::vector<uint32_t> row0, chunk0, split0;
+  std::vector<uint32_t> nheavy;  // leading chunks of band k with more than kLightOwners owners
   DBuf<Chunk> chunks;
   DBuf<SplitRow> split;
   std::vector<uint32_t> light0;  // chain schedule: the light rows of band k are
@@ -66,6 +67,7 @@ struct RowBands {
 struct ItemSet {
   const Chunk *chunks = nullptr;
   uint32_t nchunks = 0;
+  uint32_t nheavy = 0;  // leading chunks with more than kLightOwners owners (not set for the chain)
   const SplitRow *split = nullptr;
   uint32_t nsplit = 0;
   uint32_t row0 = 0, rows = 0;
@@ -94,6 +96,7 @@ struct PackedTables;
 struct TiledPlan;
 struct WarpPlan;
 struct ChainData;
+struct SplitPlan;
 
 // S3TTMc schedule: 0 = automatic (chain, else warp, else tiled, else rows),
 // 1 = per-owner rows kernel, 2 = CTA register-tiled, 3 = warp per owner,
@@ -133,6 +136,7 @@ struct TensorState {
   std::map<uint32_t, std::shared_ptr<PackedTables>> tables;  // by R
   std::map<uint32_t, std::shared_ptr<TiledPlan>> tiled;      // by R
   std::map<uint32_t, std::shared_ptr<WarpPlan>> warp;        // by R
+  std::map<uint32_t, std::shared_ptr<SplitPlan>> split_plans;  // by R
   std::unique_ptr<TreeLevels> tree;
   std::map<uint32_t, std::unique_ptr<RowBands>> bands;  // by band count
   std::shared_ptr<ChainData> chain;  // owners in pivot-chain order (s3ttmc_chain.cu)
