@@ -165,7 +165,9 @@ int symprop_unpack_rows_device(const double *dpacked, uint64_t rows,
  * full symmetric) of a device n x m row-major Y, the dense step HOOI uses
  * in place of leftsvd(Y) (src/sparse/spsymtensor.cpp:225,
  * src/dense/matrixops.cpp:18-43; symsyrk :126-146 is its n x n twin).
- * precision SYMPROP_FP64: dY, dscale are double*, FP64 CUDA-core GEMM;
+ * precision SYMPROP_FP64: dY, dscale are double*; from 1,536 rows and 320
+ * columns on integer tensor cores (exact sums of the columns rounded to 53
+ * bits of their largest entry), else FP64 CUDA-core GEMM;
  * SYMPROP_FP32: dY, dscale are float*, tcgen05 tensor cores with split-BF16
  * operands and FP32 accumulation. */
 int symprop_gram_device(const void *dY, uint64_t n, uint32_t m, const void *dscale,
@@ -331,7 +333,7 @@ int symprop_ws_predict(const symprop_tensor *t, uint32_t R, uint64_t seed, uint3
 int symprop_device_count(int *count);
 int symprop_set_device(int device);
 /* The library keeps the scratch of its dense steps (eigensolver blocks,
- * GEMM and Gram partial sums) in a per-device pool between calls, so that a
+ * GEMM and Gram partial sums, at most about 4.5 GB of an FP64 Gram's operands) in a per-device pool between calls, so that a
  * repeated solve allocates no new scratch.  This waits for the current
  * device and returns the pool's unused memory to it (memory in use is not
  * touched); call it before handing the GPU to other work.  (No reference

@@ -64,8 +64,7 @@ int symprop_set_device(int device) {
 
 int symprop_trim_memory(void) {
   return guard([&] {
-    SPB_CUDA(cudaDeviceSynchronize());
-    SPB_CUDA(cudaMemPoolTrimTo(device_pool(), 0));
+    trim_pool();
   });
 }
 

@@ -84,6 +84,11 @@ struct NvtxRange {
 
 // ---------------------------------------------------------- device buffer
 
+// The library's stream-ordered memory pool of the current device (dense.cu);
+// trim_pool waits for the device and gives it the unused memory back.
+cudaMemPool_t device_pool();
+void trim_pool();
+
 template <class T> struct DBuf {
   T *p = nullptr;
   size_t n = 0;
@@ -100,7 +105,12 @@ template <class T> struct DBuf {
   void alloc(size_t count) {
     release();
     if (count == 0) return;
-    SPB_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) {  // the pool may hold what is missing
+      cudaGetLastError();
+      p = nullptr;
+      trim_pool();
+      SPB_CUDA(cudaMalloc(&p, count * sizeof(T)));
+    }
     n = count;
   }
   // grows (never shrinks); contents are not preserved
@@ -115,8 +125,6 @@ template <class T> struct DBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
-// The library's stream-ordered memory pool of the current device (dense.cu).
-cudaMemPool_t device_pool();
 
 // ------------------------------------------------------- packed indexing
 

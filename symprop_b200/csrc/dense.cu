@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "dense.cuh"
+#include "gram_i8.cuh"
 
 namespace spb {
 namespace dense {
@@ -773,10 +774,13 @@ void gemm(cudaStream_t st, int M, int N, int K, T alpha, const T *A, int lda, bo
       SPB_LAUNCH_CHECK();
       return;
     }
-    if (transA && !transB && sym_upper && A == B && lda == ldb && M == N && !kscale && M >= GB && M % 2 == 0 &&
-        lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && alpha == 1.0 && beta == 0.0) {
-      gram_f64(st, M, K, A, lda, C, ldc);
-      return;
+    if (transA && !transB && sym_upper && A == B && lda == ldb && M == N && !kscale && alpha == 1.0 && beta == 0.0) {
+      // a column Gram: the integer tensor cores where they pay and A is finite
+      if (gram::i8_gram_pays(K, M) && gram::gram_cols_i8(st, A, K, M, lda, C, ldc)) return;
+      if (M >= GB && M % 2 == 0 && lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
+        gram_f64(st, M, K, A, lda, C, ldc);
+        return;
+      }
     }
   }
   const int tm = cdiv(M, BM), tn = cdiv(N, BN);
@@ -1076,7 +1080,8 @@ static int top_eigs_op(cudaStream_t st, const SymApply &apply, int s, int r, dou
 // the eigensolver's many small buffers cost no allocation after the first
 // iteration.  (The device's default pool releases
 // memory at every synchronisation unless its owner raised the threshold.)
-// symprop_trim_memory gives the unused part back.
+// symprop_trim_memory gives the unused part back, and so does a device buffer
+// whose allocation fails.
 cudaMemPool_t device_pool() {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
@@ -1095,6 +1100,11 @@ cudaMemPool_t device_pool() {
   SPB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
   pools[dev] = pool;
   return pool;
+}
+
+void trim_pool() {
+  SPB_CUDA(cudaDeviceSynchronize());
+  SPB_CUDA(cudaMemPoolTrimTo(device_pool(), 0));
 }
 
 }  // namespace spb

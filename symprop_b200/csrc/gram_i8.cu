@@ -1,0 +1,504 @@
+// FP64 column Gram C = A^T A on the 8-bit integer tensor cores (tcgen05
+// kind::i8): HOOI's dense step in FP64 (src/sparse/spsymtensor.cpp:225,
+// src/dense/matrixops.cpp:18-43 form it with LAPACK).
+//
+// Method: Ozaki scheme II (Ozaki, Uchino, Imamura 2025), a matrix product of
+// integers by the Chinese remainder theorem.  The rows are taken in chunks of
+// at most kMaxChunk.  In a chunk every column is scaled by a power of two so
+// that its largest magnitude is in [2^52, 2^53) and rounded to integers,
+//     a_kj = 2^-s_j n_kj + delta,  |delta| <= 2^-s_j / 2  (exact to 2^-53 of
+//     the column's largest entry of the chunk),
+// and sum_k n_ki n_kj, an integer of at most 2^122, is found from its residues
+// modulo 16 pairwise coprime p <= 256 (product 2^125.4): residues of the n_kj
+// fit 8 bits, each modulus is one int8 product with exact int32 sums
+// (at most chunk * 2^14 = 2^30), and the sum is put together in 128-bit integers and
+// rounded once.  The chunks' sums are added in FP64.  No accumulation error
+// grows with the number of rows: the error is that of the scaled rounding,
+// 2^-54 of the column maximum per entry with random sign, and of one rounding
+// per chunk.
+//
+// Bound: 16 int8 products over the upper 256 x 256 tiles.  200,000 x 3,876:
+// 136 tiles, 5.7e13 integer operations (12.7 ms at the nominal 4.5 POP/s),
+// against 3.0e12 FP64 operations (81 ms at the nominal 37 TFLOP/s) for the
+// CUDA-core kernel in dense.cu (137 ms).  Measured 27.6 ms: product 17.9 (3.2
+// POP/s), residues 5.8 (reads A, writes 16 bytes per entry), remainders 1.1,
+// column maxima 0.9; error against 64 bits 1.2e-16, 6.2e-15 for the CUDA-core
+// kernel.  Running the residues and remainders on a second stream beside the
+// product gave nothing (29.0 against 28.9 ms).
+//
+// Kernel (i8_gram_kernel): one CTA of 256 threads per (tile, modulus, chunk),
+// 256 x 256 outputs as two M = 128, N = 256 accumulators that fill the tensor
+// memory (64 KB of operands per 128-wide k block and 1024 tensor clocks: the
+// 128 x 256 tile of gram_tc.cu would read 1.5 times as much of them from L2).
+// Warp 0 loads (TMA, 128-byte swizzle, 3 stages), warp 1 issues, all 8 warps
+// reduce the sums modulo p and store one byte per entry.  Waits are bounded
+// as in gram_tc.cu.
+#include <algorithm>
+#include <cmath>
+
+#include "gram_i8.cuh"
+#include "gram_tc.cuh"
+#include "tcgen05.cuh"
+
+namespace spb {
+namespace gram {
+namespace {
+
+constexpr int kP = 16;
+constexpr int kModulus[kP] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
+constexpr int kMaxChunk = 65536;  // rows: 2^16 * 2^106 < P / 8 and 2^16 * 2^14 = 2^30
+constexpr int kTile = 256, kBK = 128, kNStages = 3;
+constexpr uint32_t kOperand = kTile * kBK;  // bytes
+constexpr size_t kSmem = (size_t)kNStages * 2 * kOperand + 1024;
+
+// (P / p)^-1 mod p of every modulus, and P / p and P as two 64-bit words
+struct Crt {
+  uint32_t inv[kP];
+  unsigned long long wlo[kP], whi[kP], plo, phi;
+  double rp[kP];  // 1 / p
+};
+
+constexpr Crt make_crt() {
+  Crt t{};
+  unsigned __int128 P = 1;
+  for (int i = 0; i < kP; ++i) P *= (unsigned)kModulus[i];
+  t.plo = (unsigned long long)P;
+  t.phi = (unsigned long long)(P >> 64);
+  for (int i = 0; i < kP; ++i) {
+    const unsigned p = (unsigned)kModulus[i];
+    const unsigned __int128 w = P / p;
+    t.wlo[i] = (unsigned long long)w;
+    t.whi[i] = (unsigned long long)(w >> 64);
+    const unsigned r = (unsigned)(w % p);
+    for (unsigned x = 1; x < p; ++x)
+      if (r * x % p == 1) t.inv[i] = x;
+    t.rp[i] = 1.0 / p;
+  }
+  return t;
+}
+__constant__ Crt c_crt = make_crt();
+__constant__ int c_mod[kP] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
+
+// ------------------------------------------------------------ preparation
+
+// Bits of the largest magnitude of every column of every chunk (magnitudes
+// order as integers; an infinity or a NaN comes out on top)
+__global__ void __launch_bounds__(128) col_max_kernel(const double *__restrict__ A, int rows, int cols, int lda,
+                                                      int chunk, int part, unsigned long long *__restrict__ cmax) {
+  const int c = blockIdx.x * 128 + threadIdx.x;
+  const int k0 = blockIdx.y * chunk + blockIdx.z * part, k1 = min(min(rows, (int)(blockIdx.y + 1) * chunk), k0 + part);
+  if (c >= cols || k0 >= k1) return;
+  unsigned long long m = 0;
+#pragma unroll 8
+  for (int k = k0; k < k1; ++k) m = max(m, __double_as_longlong(A[(size_t)k * lda + c]) & 0x7fffffffffffffffull);
+  atomicMax(&cmax[(size_t)blockIdx.y * cols + c], m);
+}
+
+// Exponent s of every column: |a| 2^s < 2^53; *bad is set when one is not finite
+__global__ void scale_kernel(const unsigned long long *cmax, int n, int *s, int *bad) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const unsigned long long b = cmax[i];
+  if (b >= 0x7ff0000000000000ull) *bad = 1;
+  int e = 0;
+  if (b) frexp(__longlong_as_double((long long)b), &e);  // |a| < 2^e
+  s[i] = b ? 53 - e : 0;
+}
+
+// Residues of the scaled columns: out[(chunk * 16 + p) * cols + c][k], k < kc
+// bytes contiguous (rows past the chunk's end are zero).  A thread takes 32
+// rows of one column: a warp reads 256-byte row pieces, and every store fills a
+// 32-byte sector.  q = round(n / p) is within 2^-7 of n / p + 1/2, so |r| may
+// pass p / 2 by 2: put back into 8 bits where p / 2 + 2 > 127.
+__global__ void __launch_bounds__(128) residue_kernel(const double *__restrict__ A, int rows, int cols, int lda,
+                                                      int chunk, int kc, const int *__restrict__ s, int chunk0,
+                                                      signed char *__restrict__ out) {
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31);
+  const int k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 32;  // within the chunk
+  if (c >= cols) return;
+  const int ch = chunk0 + blockIdx.z;
+  const int r0 = ch * chunk + k0, r1 = min(rows, (ch + 1) * chunk);
+  const int sh = s[(size_t)ch * cols + c], s1 = sh / 2;
+  // 2^sh as two factors: sh may lie outside the exponent range
+  const double f1 = __longlong_as_double((long long)(s1 + 1023) << 52),
+               f2 = __longlong_as_double((long long)(sh - s1 + 1023) << 52);
+  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+  double n[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) n[i] = r0 + i < r1 ? rint(A[(size_t)(r0 + i) * lda + c] * f1 * f2) : 0.0;
+  for (int p = 0; p < kP; ++p) {
+    const double m = (double)c_mod[p], rm = c_crt.rp[p];
+    uint32_t w[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      uint32_t v = 0;
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const double x = n[4 * q + b];
+        const double t = fma(x, rm, kMagic) - kMagic;
+        int r = (int)__double_as_longlong(fma(-t, m, x) + kMagic);  // the low word holds the integer
+        if (p == 1 || p == 2) {  // 255, 253 (for 256 the byte wraps to the same residue)
+          const int mi = c_mod[p];
+          r = r > 127 ? r - mi : r < -128 ? r + mi : r;
+        }
+        v |= (uint32_t)(r & 0xff) << (8 * b);
+      }
+      w[q] = v;
+    }
+    uint4 *o = reinterpret_cast<uint4 *>(out + ((size_t)(blockIdx.z * kP + p) * cols + c) * kc + k0);
+    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
+// ---------------------------------------------------------------- product
+
+constexpr uint32_t kIdesc = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTile >> 3) << 17) | ((128u >> 4) << 24);
+
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t acc) {
+  uint32_t z = 0;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}" ::"r"(tmem_d),
+      "l"(da), "l"(db), "r"(kIdesc), "r"(acc), "r"(z), "r"(z), "r"(z), "r"(z));
+}
+
+struct I8Args {
+  int cols, ntile, ntiles;    // tiles of 256 per side, upper tiles
+  int kblocks;                // 128-wide blocks of a chunk
+  unsigned char *C;           // (chunk * 16 + p) planes of ld x ld residues
+  int ld;
+  int *err;
+  uint64_t wait_ns;
+};
+
+__global__ void __launch_bounds__(256, 1)
+    i8_gram_kernel(const __grid_constant__ CUtensorMap map, const I8Args a) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  __shared__ __align__(8) uint64_t full_bar[kNStages], empty_bar[kNStages], done_bar;
+  __shared__ uint32_t tmem_base_holder;
+  __shared__ volatile int abort_flag;
+  __shared__ volatile int progress;
+  __shared__ int issued[kNStages];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // unit: tile fastest, so that the CTAs of a wave share a modulus in L2
+  const int plane = (int)blockIdx.x / a.ntiles;
+  int ti = 0, tj = (int)blockIdx.x - plane * a.ntiles;
+  while (tj >= a.ntile - ti) {
+    tj -= a.ntile - ti;
+    ++ti;
+  }
+  tj += ti;
+  const int row0 = plane * a.cols + ti * kTile, col0 = plane * a.cols + tj * kTile;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kNStages; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+      issued[s] = 0;
+    }
+    mbar_init(&done_bar, 1);
+    abort_flag = 0;
+    progress = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
+                     smem_u32(&tmem_base_holder)),
+                 "r"(512u));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_base_holder;
+
+  if (warp == 0 && lane == 0) {
+    for (int it = 0; it < a.kblocks; ++it) {
+      const int s = it % kNStages;
+      const uint32_t round = (uint32_t)(it / kNStages);
+      if (it >= kNStages && !mbar_wait(&empty_bar[s], (round - 1) & 1, &abort_flag, a.wait_ns)) {
+        abort_flag = 1;
+        break;
+      }
+      unsigned char *st = smem + (size_t)s * 2 * kOperand;
+      mbar_expect_tx(&full_bar[s], 2 * kOperand);
+      tma_load_2d(st, &map, &full_bar[s], it * kBK, row0);
+      tma_load_2d(st + kOperand, &map, &full_bar[s], it * kBK, col0);
+      issued[s] = it + 1;
+    }
+  } else if (warp == 1 && lane == 0) {
+    bool ok = true;
+    for (int it = 0; it < a.kblocks; ++it) {
+      const int s = it % kNStages;
+      if (!mbar_wait(&full_bar[s], (uint32_t)(it / kNStages) & 1, &abort_flag, a.wait_ns)) {
+        abort_flag = 1;
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t base = smem_u32(smem + (size_t)s * 2 * kOperand);
+#pragma unroll
+      for (int k = 0; k < kBK / 32; ++k) {  // K-major rows of 128 bytes, 32 bytes a step
+        const uint64_t db = smem_desc(base + kOperand + k * 32, 16u);
+        umma_i8(tmem, smem_desc(base + k * 32, 16u), db, (it > 0 || k > 0) ? 1u : 0u);
+        umma_i8(tmem + 256u, smem_desc(base + 128 * kBK + k * 32, 16u), db, (it > 0 || k > 0) ? 1u : 0u);
+      }
+      umma_commit(&empty_bar[s]);
+      progress = it + 1;
+    }
+    umma_commit(&done_bar);
+    if (!ok) abort_flag = 1;
+  }
+  __syncwarp();
+  const bool done = mbar_wait_progress(&done_bar, &progress);
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const int go = __all_sync(0xffffffffu, done ? 1 : 0) && !__shfl_sync(0xffffffffu, (int)abort_flag, 0);
+  if (go) {
+    // warp w: lanes of quadrant w % 4 of accumulator w / 4.  The sums (at most
+    // 2^30 in magnitude) modulo p, times (P / p)^-1 modulo p.
+    const int half = warp >> 2, r = ti * kTile + half * 128 + (warp & 3) * 32 + lane;
+    const uint32_t p = (uint32_t)c_mod[plane % kP], inv = c_crt.inv[plane % kP];
+    const uint32_t magic = 0xffffffffu / p, bias = (1u << 30) / p * p + p;
+    unsigned char *C = a.C + (size_t)plane * a.ld * a.ld + (size_t)r * a.ld + tj * kTile;
+#pragma unroll 1
+    for (int c = 0; c < kTile; c += 32) {
+      uint32_t v[32];
+      tmem_load<32>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * 256 + c), v);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      uint32_t o[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        o[q] = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          uint32_t u = v[4 * q + b] + bias;  // the sum plus a multiple of p, positive
+          u -= __umulhi(u, magic) * p;       // below 2 p + small: at most two subtractions
+          u = u >= p ? u - p : u;
+          u = u >= p ? u - p : u;
+          u *= inv;
+          u -= __umulhi(u, magic) * p;
+          u = u >= p ? u - p : u;
+          u = u >= p ? u - p : u;
+          o[q] |= u << (8 * b);
+        }
+      }
+      uint4 *d = reinterpret_cast<uint4 *>(C + c);  // rows up to ld are stored: ld is a multiple of 256
+      d[0] = make_uint4(o[0], o[1], o[2], o[3]);
+      d[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    }
+  } else if (threadIdx.x == 0) {
+    atomicExch(a.err, 1);
+  }
+  if (threadIdx.x == 0 && (abort_flag || !done)) {
+    for (int s = 0; s < kNStages; ++s)
+      if (issued[s] > 0) {
+        volatile int never = 0;
+        mbar_wait(&full_bar[s], (uint32_t)((issued[s] - 1) / kNStages) & 1, &never, kWaitNs);
+      }
+    if (!done) {
+      volatile int never = 0;
+      mbar_wait(&done_bar, 0, &never, kWaitNs);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (warp == 0)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+}
+
+// ------------------------------------------------------------- remainders
+
+// One 32 x 32 tile (i0 <= j0) of C and its mirror image: every chunk's sum
+// X = sum_p c_p (P / p) - P round(sum_p c_p / p) in 128 bits (|X| < P / 8, so the
+// rounding is never in doubt), scaled back and added in FP64, chunks in order.
+__global__ void __launch_bounds__(256) crt_kernel(const unsigned char *__restrict__ R, int ld, int cols, int nchunk,
+                                                  int chunk0, const int *__restrict__ s, int add,
+                                                  double *__restrict__ C, int ldc) {
+  if (blockIdx.x < blockIdx.y) return;
+  __shared__ double t[32][33];
+  const int j0 = blockIdx.x * 32, i0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const size_t pl = (size_t)ld * ld;
+#pragma unroll 1
+  for (int y = ty; y < 32; y += 8) {
+    const int i = i0 + y, j = j0 + tx;
+    double sum = 0.0;
+    if (i < cols && j < cols) {
+      if (add) sum = C[(size_t)i * ldc + j];
+      for (int c = 0; c < nchunk; ++c) {
+        const unsigned char *r = R + (size_t)c * kP * pl + (size_t)i * ld + j;
+        unsigned long long lo = 0, hi = 0;
+        double q = 0.0;
+#pragma unroll
+        for (int p = 0; p < kP; ++p) {
+          const unsigned long long v = r[p * pl], x = v * c_crt.wlo[p];
+          lo += x;
+          hi += v * c_crt.whi[p] + __umul64hi(v, c_crt.wlo[p]) + (lo < x ? 1ull : 0ull);
+          q += (double)v * c_crt.rp[p];
+        }
+        const unsigned long long k = (unsigned long long)rint(q), x = k * c_crt.plo;
+        hi -= k * c_crt.phi + __umul64hi(k, c_crt.plo) + (lo < x ? 1ull : 0ull);
+        lo -= x;
+        const bool neg = (long long)hi < 0;
+        if (neg) {
+          lo = ~lo + 1;
+          hi = ~hi + (lo == 0 ? 1ull : 0ull);
+        }
+        // hi < 2^60: bring the value to 64 bits plus a sticky bit, so that one
+        // conversion rounds it
+        int sh = 0;
+        if (hi) {
+          sh = 64 - __clzll((long long)hi);
+          const unsigned long long rest = lo << (64 - sh);
+          lo = (sh < 64 ? (hi << (64 - sh)) | (lo >> sh) : hi) | (rest ? 1ull : 0ull);
+        }
+        const double d = (double)lo;
+        sum += scalbn(neg ? -d : d, sh - s[(size_t)(chunk0 + c) * cols + i] - s[(size_t)(chunk0 + c) * cols + j]);
+      }
+      if (i <= j) C[(size_t)i * ldc + j] = sum;
+    }
+    t[y][tx] = sum;
+  }
+  __syncthreads();
+  for (int y = ty; y < 32; y += 8) {  // the mirror image: row j0 + y, column i0 + tx
+    const int j = j0 + y, i = i0 + tx;
+    if (i < j && j < cols) C[(size_t)j * ldc + i] = t[tx][y];
+  }
+}
+
+int sms() {
+  int dev = 0, n = 0;
+  SPB_CUDA(cudaGetDevice(&dev));
+  SPB_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+  return std::max(n, 1);
+}
+
+// Chunks of the rows.  A product takes 1024 clocks per 128 rows and about
+// 12,000 besides (loads of the first stages, reduction, tensor memory), one
+// per SM at a time: of the chunk counts the one whose waves take least, as
+// long as the chunks launched together stay within kGroupBytes.
+constexpr size_t kGroupBytes = 9ull << 29;  // 4.5 GB of residues and remainders
+struct I8Plan {
+  int ntile, ntiles, ld;
+  int chunk, nchunk;  // rows per chunk
+  int kc, group;      // padded rows, chunks per launch
+};
+
+I8Plan plan_i8(int rows, int cols) {
+  I8Plan g;
+  g.ntile = (cols + kTile - 1) / kTile;
+  g.ntiles = g.ntile * (g.ntile + 1) / 2;
+  g.ld = g.ntile * kTile;
+  const int n = sms();
+  const int c0 = (rows + kMaxChunk - 1) / kMaxChunk;
+  double best = 1e300;
+  for (int c = c0; c <= std::max(c0, std::min(c0 + 24, rows / 1024)); ++c) {
+    const int kc = ((rows + c - 1) / c + kBK - 1) / kBK * kBK;
+    const size_t bytes = (size_t)kP * ((size_t)cols * kc + (size_t)g.ld * g.ld);
+    const int group = (int)std::max<size_t>(1, std::min<size_t>((size_t)c, kGroupBytes / bytes));
+    double t = 0;
+    for (int x = 0; x < c; x += group) {
+      const double units = (double)g.ntiles * kP * std::min(group, c - x);
+      t += std::ceil(units / n) * (kc / kBK * 1024.0 + 12000.0);
+    }
+    if (t < best) {
+      best = t;
+      g.chunk = kc;
+      g.nchunk = (rows + kc - 1) / kc;
+      g.kc = kc;
+      g.group = group;
+    }
+  }
+  g.group = std::min(g.group, g.nchunk);
+  return g;
+}
+
+struct Pool {  // scratch from the library's stream-ordered pool
+  void *p = nullptr;
+  cudaStream_t st;
+  explicit Pool(cudaStream_t s) : st(s) {}
+  Pool(size_t bytes, cudaStream_t s) : st(s) {
+    SPB_CUDA(cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 256), device_pool(), st));
+  }
+  bool take_operands(size_t bytes) {  // false when the device has not that much left
+    if (cudaMallocFromPoolAsync(&p, bytes, device_pool(), st) == cudaSuccess) return true;
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
+  ~Pool() {
+    if (p) cudaFreeAsync(p, st);
+  }
+};
+
+}  // namespace
+
+// Six launches, two waits and 256-wide tiles are paid back from about 1,500 rows
+// on (2,000 x 816: 0.43 -> 0.19 ms, 2,000 x 3,876: 1.73 -> 1.01 ms; 1,024 x
+// 2,002: 0.27 -> 0.31 ms) and from about 320 columns (10,000 x 256: 0.28 ms
+// either way).
+bool i8_gram_pays(int rows, int cols) { return cols >= 320 && rows >= 1536; }
+
+bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc) {
+  const I8Plan g = plan_i8(rows, cols);
+  const size_t ncs = (size_t)g.nchunk * cols;
+  Pool cmax(ncs * 8, st), sc(ncs * 4, st), flags(2 * sizeof(int), st);
+  int *bad = (int *)flags.p, *err = bad + 1;
+  SPB_CUDA(cudaMemsetAsync(cmax.p, 0, ncs * 8, st));
+  SPB_CUDA(cudaMemsetAsync(flags.p, 0, 2 * sizeof(int), st));
+  const int part = 512;
+  col_max_kernel<<<dim3((cols + 127) / 128, g.nchunk, (g.chunk + part - 1) / part), 128, 0, st>>>(
+      A, rows, cols, lda, g.chunk, part, (unsigned long long *)cmax.p);
+  SPB_LAUNCH_CHECK();
+  scale_kernel<<<(unsigned)((ncs + 255) / 256), 256, 0, st>>>((const unsigned long long *)cmax.p, (int)ncs,
+                                                              (int *)sc.p, bad);
+  SPB_LAUNCH_CHECK();
+  int h[2] = {0, 0};
+  SPB_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SPB_CUDA(cudaStreamSynchronize(st));
+  if (h[0]) return false;
+  SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+  Pool res(st), rem(st);
+  if (!res.take_operands((size_t)g.group * kP * cols * g.kc) || !rem.take_operands((size_t)g.group * kP * g.ld * g.ld))
+    return false;
+  for (int c0 = 0; c0 < g.nchunk; c0 += g.group) {
+    const int nc = std::min(g.group, g.nchunk - c0);
+    residue_kernel<<<dim3((cols + 31) / 32, g.kc / 128, nc), 128, 0, st>>>(A, rows, cols, lda, g.chunk, g.kc,
+                                                                          (const int *)sc.p, c0,
+                                                                          (signed char *)res.p);
+    SPB_LAUNCH_CHECK();
+    CUtensorMap map;
+    cuuint64_t dims[2] = {(cuuint64_t)g.kc, (cuuint64_t)nc * kP * cols};
+    cuuint64_t strides[1] = {(cuuint64_t)g.kc};
+    cuuint32_t box[2] = {kBK, kTile}, estr[2] = {1, 1};
+    const CUresult r = get_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, res.p, dims, strides, box, estr,
+                                     CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) fail(SYMPROP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+    I8Args a;
+    a.cols = cols;
+    a.ntile = g.ntile;
+    a.ntiles = g.ntiles;
+    a.kblocks = g.kc / kBK;
+    a.C = (unsigned char *)rem.p;
+    a.ld = g.ld;
+    a.err = err;
+    a.wait_ns = mainloop_wait_ns();
+    i8_gram_kernel<<<(unsigned)(g.ntiles * kP * nc), 256, kSmem, st>>>(map, a);
+    SPB_LAUNCH_CHECK();
+    const unsigned nt = (unsigned)((cols + 31) / 32);
+    crt_kernel<<<dim3(nt, nt), 256, 0, st>>>((const unsigned char *)rem.p, g.ld, cols, nc, c0, (const int *)sc.p,
+                                             c0 > 0 ? 1 : 0, C, ldc);
+    SPB_LAUNCH_CHECK();
+  }
+  SPB_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+  SPB_CUDA(cudaStreamSynchronize(st));
+  if (h[1]) fail(SYMPROP_ERR_TIMEOUT, "integer tensor-core Gram: a bounded wait expired");
+  return true;
+}
+
+}  // namespace gram
+}  // namespace spb
