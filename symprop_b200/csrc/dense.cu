@@ -28,62 +28,78 @@ inline unsigned cdiv(long long a, long long b) { return (unsigned)((a + b - 1) /
 
 // ------------------------------------------------------------------- GEMM
 
-constexpr int BM = 64, BN = 64, BK = 16;
+// 64 x NB tiles (NB = 64, or 32 for products of at most 32 columns), k blocks
+// of 16 in two shared buffers: the next block's loads are in flight during the
+// current one, one barrier per block.
+constexpr int BM = 64, BK = 16;
 
-template <typename T, bool TA, bool TB, bool KS>
+template <typename T, int NB, bool TA, bool TB, bool KS>
 __global__ void __launch_bounds__(256) gemm_tile_kernel(int M, int N, int K, const T *__restrict__ A,
                                                         int lda, const T *__restrict__ B, int ldb,
                                                         const T *__restrict__ ks, T *out, int ldo,
                                                         int kchunk, int sym_upper,
                                                         size_t split_stride) {
   const int tm = blockIdx.y, tn = blockIdx.x;
-  if (sym_upper && tm > tn) return;
-  const int bm = tm * BM, bn = tn * BN;
+  if (sym_upper && tm * BM >= (tn + 1) * NB) return;  // below the diagonal
+  constexpr int EA = BM * BK / 256, EB = NB * BK / 256, CN = NB / 16;
+  const int bm = tm * BM, bn = tn * NB;
   const int k0 = blockIdx.z * kchunk;
   const int k1 = min(K, k0 + kchunk);
-  __shared__ T As[BK][BM + 1];
-  __shared__ T Bs[BK][BN + 1];
+  __shared__ T As[2][BK][BM + 1];
+  __shared__ T Bs[2][BK][NB + 1];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  T acc[4][4];
+  T ra[EA], rb[EB];
+  auto fetch = [&](int kk) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = T(0);
-  for (int kk = k0; kk < k1; kk += BK) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      int idx = tid + e * 256;
-      int kq, im;
-      if (TA) { kq = idx / BM; im = idx % BM; } else { im = idx / BK; kq = idx % BK; }
-      int gi = bm + im, gk = kk + kq;
+    for (int e = 0; e < EA; ++e) {
+      const int idx = tid + e * 256, kq = TA ? idx / BM : idx % BK, im = TA ? idx % BM : idx / BK;
+      const int gi = bm + im, gk = kk + kq;
       T v = T(0);
       if (gi < M && gk < k1) {
         v = TA ? A[(size_t)gk * lda + gi] : A[(size_t)gi * lda + gk];
         if (KS) v *= ks[gk];
       }
-      As[kq][im] = v;
-      int jn;
-      if (TB) { jn = idx / BK; kq = idx % BK; } else { kq = idx / BN; jn = idx % BN; }
-      int gj = bn + jn;
-      gk = kk + kq;
-      T w = T(0);
-      if (gj < N && gk < k1) w = TB ? B[(size_t)gj * ldb + gk] : B[(size_t)gk * ldb + gj];
-      Bs[kq][jn] = w;
+      ra[e] = v;
+    }
+#pragma unroll
+    for (int e = 0; e < EB; ++e) {
+      const int idx = tid + e * 256, kq = TB ? idx % BK : idx / NB, jn = TB ? idx / BK : idx % NB;
+      const int gj = bn + jn, gk = kk + kq;
+      rb[e] = gj < N && gk < k1 ? (TB ? B[(size_t)gj * ldb + gk] : B[(size_t)gk * ldb + gj]) : T(0);
+    }
+  };
+  T acc[4][CN];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < CN; ++j) acc[i][j] = T(0);
+  if (k0 < k1) fetch(k0);
+  int buf = 0;
+  for (int kk = k0; kk < k1; kk += BK, buf ^= 1) {
+#pragma unroll
+    for (int e = 0; e < EA; ++e) {
+      const int idx = tid + e * 256;
+      As[buf][TA ? idx / BM : idx % BK][TA ? idx % BM : idx / BK] = ra[e];
+    }
+#pragma unroll
+    for (int e = 0; e < EB; ++e) {
+      const int idx = tid + e * 256;
+      Bs[buf][TB ? idx % BK : idx / NB][TB ? idx / BK : idx % NB] = rb[e];
     }
     __syncthreads();
+    if (kk + BK < k1) fetch(kk + BK);
 #pragma unroll
     for (int kq = 0; kq < BK; ++kq) {
-      T a[4], b[4];
+      T a[4], b[CN];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kq][ty * 4 + i];
+      for (int i = 0; i < 4; ++i) a[i] = As[buf][kq][ty * 4 + i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kq][tx * 4 + j];
+      for (int j = 0; j < CN; ++j) b[j] = Bs[buf][kq][tx * CN + j];
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] += a[i] * b[j];
+        for (int j = 0; j < CN; ++j) acc[i][j] += a[i] * b[j];
     }
-    __syncthreads();
   }
   T *o = out + blockIdx.z * split_stride;
 #pragma unroll
@@ -91,8 +107,8 @@ __global__ void __launch_bounds__(256) gemm_tile_kernel(int M, int N, int K, con
     int gi = bm + ty * 4 + i;
     if (gi >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      int gj = bn + tx * 4 + j;
+    for (int j = 0; j < CN; ++j) {
+      int gj = bn + tx * CN + j;
       if (gj < N) o[(size_t)gi * ldo + gj] = acc[i][j];
     }
   }
@@ -478,113 +494,192 @@ __global__ void __launch_bounds__(1024) householder_kernel(double *A, int rows, 
 
 // --------------------------------------------------------------- Jacobi
 
-__global__ void __launch_bounds__(1024) jacobi_kernel(const double *S, int n, double *w_out,
-                                                      double *V_out) {
-  extern __shared__ double sm[];
-  const int np = (n + 1) & ~1;
-  const int ld = np + 1;     // odd row stride: column sweeps hit distinct banks
-  double *A = sm;            // np x ld
-  double *V = sm + np * ld;  // np x ld
-  __shared__ double cs[2 * 64];
-  __shared__ int pr[2 * 64];
-  __shared__ int order[128];
-  __shared__ double red[1024];
+// Cyclic Jacobi with the round-robin pairing (np - 1 steps of np / 2 disjoint
+// pairs a sweep), in two kernels:
+//   jacobi_kernel  one CTA: the upper triangle of A in shared memory.  Per step
+//                  np / 2 threads form the rotations, then a thread per pair of
+//                  rotations (k <= l) updates the 2 x 2 block of A that they
+//                  share, rows and columns at once: two barriers a step.  The
+//                  rotations go to memory.
+//   jacobi_vectors_kernel  V = product of the rotations: its rows are
+//                  independent, one warp each.
+// Bound by latency: a step is a chain of a few hundred cycles (rotation,
+// barrier, block, barrier) whatever n is.  n = 96: 2.75 ms with rows,
+// columns and V updated in turn by one CTA (four barriers a step, a serial
+// sort), 0.92 + 0.19 ms now; n = 64: 1.04 -> 0.39 + 0.09 ms.
+constexpr int kJacobiSweeps = 60;
+
+// the pair of place k at a step: indices p < q
+__device__ __forceinline__ void jacobi_pair(int k, int step, int np, int &p, int &q) {
+  int a = k + step;  // 1 + (k - 1 + step) mod (np - 1), k >= 1
+  a = k == 0 ? 0 : a >= np ? a - (np - 1) : a;
+  int b = np - 1 - k + step;
+  b = b >= np ? b - (np - 1) : b;
+  p = min(a, b);
+  q = max(a, b);
+}
+
+// w_out: eigenvalues, descending; place[j]: place of index j among them;
+// rot: (c, s) of every pair of every step; *sweeps: how many were done
+__global__ void __launch_bounds__(1024) jacobi_kernel(const double *S, int n, double *w_out, double2 *rot, int *place,
+                                                      int *sweeps) {
+  extern __shared__ double A[];  // np x ld, upper triangle
+  const int np = (n + 1) & ~1, half = np / 2;
+  const int ld = np + 1;  // odd row stride: column reads fall on different banks
+  __shared__ double2 cs[kJacobiMax / 2];
+  __shared__ int2 pr[kJacobiMax / 2];
+  __shared__ double red[33];
   __shared__ int rotated;
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nwarp = nt >> 5;
-  for (int idx = tid; idx < np * np; idx += nt) {
-    int i = idx / np, j = idx % np;
-    A[i * ld + j] = (i < n && j < n) ? S[i * n + j] : 0.0;
-    V[i * ld + j] = (i == j) ? 1.0 : 0.0;
-  }
+  const int tid = threadIdx.x, nt = blockDim.x;
+  // scaled by a power of two to entries of at most 1
+  double mx = 0.0;
+  for (int idx = tid; idx < n * n; idx += nt) mx = fmax(mx, fabs(S[idx]));
+  for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((tid & 31) == 0) red[tid >> 5] = mx;
   __syncthreads();
-  double fro = 0;
+  for (int w = 0; w < nt / 32; ++w) mx = fmax(mx, red[w]);
+  __syncthreads();
+  int e = 0;
+  if (mx > 0.0 && isfinite(mx)) frexp(mx, &e);
+  double fro = 0.0;
   for (int idx = tid; idx < np * np; idx += nt) {
-    const double x = A[(idx / np) * ld + idx % np];
+    const int i = idx / np, j = idx % np;
+    const double x = i < n && j < n ? scalbn(S[i * n + j], -e) : 0.0;
     fro += x * x;
+    if (i <= j) A[i * ld + j] = x;
   }
   fro = block_sum(fro, red);
-  const int half = np / 2;
-  for (int sweep = 0; sweep < 60 && np > 1; ++sweep) {
-    double off = 0;
-    for (int idx = tid; idx < np * np; idx += nt) {
-      int i = idx / np, j = idx % np;
-      if (i != j) off += A[i * ld + j] * A[i * ld + j];
+  const double tiny = 1e-18 * sqrt(fro);
+  // this thread's blocks: pairs (k, l) of rotations, k <= l
+  constexpr int kBlk = 2;  // 48 * 49 / 2 over at least 588 threads
+  const int nblk = half * (half + 1) / 2;
+  int bk[kBlk], bl[kBlk];
+#pragma unroll
+  for (int t = 0; t < kBlk; ++t) {
+    int k = 0, r = tid + t * nt;
+    bk[t] = -1;
+    bl[t] = 0;
+    if (r < nblk) {
+      while (r >= half - k) {
+        r -= half - k;
+        ++k;
+      }
+      bk[t] = k;
+      bl[t] = k + r;
     }
-    off = block_sum(off, red);
+  }
+  int sweep = 0;
+  for (; sweep < kJacobiSweeps && np > 1; ++sweep) {
+    double off = 0.0;
+    for (int idx = tid; idx < np * np; idx += nt) {
+      const int i = idx / np, j = idx % np;
+      if (i < j) off += A[i * ld + j] * A[i * ld + j];
+    }
+    off = 2.0 * block_sum(off, red);
     if (!(off > 1e-30 * fro)) break;
     if (tid == 0) rotated = 0;
     __syncthreads();
     for (int step = 0; step < np - 1; ++step) {
       if (tid < half) {
-        int k = tid;
-        int a = (k == 0) ? 0 : 1 + (k - 1 + step) % (np - 1);
-        int kb = np - 1 - k;
-        int b = 1 + (kb - 1 + step) % (np - 1);
-        int p = min(a, b), q = max(a, b);
-        pr[2 * k] = p;
-        pr[2 * k + 1] = q;
+        int p, q;
+        jacobi_pair(tid, step, np, p, q);
         const double apq = A[p * ld + q], app = A[p * ld + p], aqq = A[q * ld + q];
-        double c = 1.0, s = 0.0;
+        double c = 1.0, sn = 0.0;
         // an element below the rounding level of its diagonal pair (or of
         // the whole matrix) is left alone; a sweep that rotates nothing ends
         // the iteration (rounding noise keeps off() from reaching zero)
-        const bool negligible = fabs(apq) <= 1e-17 * sqrt(fabs(app * aqq)) || fabs(apq) <= 1e-18 * sqrt(fro);
-        if (!negligible) {
+        if (!(apq * apq <= 1e-34 * fabs(app * aqq) || fabs(apq) <= tiny)) {
           rotated = 1;
-          double tau = (aqq - app) / (2.0 * apq);
-          double t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-          c = 1.0 / sqrt(1.0 + t * t);
-          s = t * c;
+          // the tangent needs few digits (what it leaves of apq, 1e-7 of it, is
+          // the next sweep's); the rotation must be orthogonal to the last one
+          const float tau = (float)(aqq - app) / (float)(2.0 * apq);
+          const double t = (double)((tau >= 0.f ? 1.f : -1.f) / (fabsf(tau) + sqrtf(1.f + tau * tau)));
+          c = rsqrt(fma(t, t, 1.0));
+          sn = t * c;
         }
-        cs[2 * k] = c;
-        cs[2 * k + 1] = s;
+        cs[tid] = make_double2(c, sn);
+        pr[tid] = make_int2(p, q);
+        rot[((size_t)sweep * (np - 1) + step) * half + tid] = make_double2(c, sn);
       }
       __syncthreads();
-      // warp w applies rotations w, w+32, ...; its lanes stride the rows or
-      // columns (no integer division in the sweep)
-      for (int k = warp; k < half; k += nwarp) {  // rows: A <- J^T A
-        const int p = pr[2 * k], q = pr[2 * k + 1];
-        const double c = cs[2 * k], s = cs[2 * k + 1];
-        for (int col = lane; col < np; col += 32) {
-          const double a = A[p * ld + col], b = A[q * ld + col];
-          A[p * ld + col] = c * a - s * b;
-          A[q * ld + col] = s * a + c * b;
-        }
-      }
-      __syncthreads();
-      for (int k = warp; k < half; k += nwarp) {  // cols: A <- A J, V <- V J
-        const int p = pr[2 * k], q = pr[2 * k + 1];
-        const double c = cs[2 * k], s = cs[2 * k + 1];
-        for (int row = lane; row < np; row += 32) {
-          const double a = A[row * ld + p], b = A[row * ld + q];
-          A[row * ld + p] = c * a - s * b;
-          A[row * ld + q] = s * a + c * b;
-          const double va = V[row * ld + p], vb = V[row * ld + q];
-          V[row * ld + p] = c * va - s * vb;
-          V[row * ld + q] = s * va + c * vb;
-        }
+#pragma unroll
+      for (int t = 0; t < kBlk; ++t) {
+        if (bk[t] < 0) continue;
+        const double2 u = cs[bk[t]], v = cs[bl[t]];
+        if (u.y == 0.0 && v.y == 0.0) continue;
+        const int2 r = pr[bk[t]], c = pr[bl[t]];
+        double *x00 = A + min(r.x, c.x) * ld + max(r.x, c.x), *x01 = A + min(r.x, c.y) * ld + max(r.x, c.y),
+               *x10 = A + min(r.y, c.x) * ld + max(r.y, c.x), *x11 = A + min(r.y, c.y) * ld + max(r.y, c.y);
+        const double a00 = *x00, a01 = *x01, a10 = *x10, a11 = *x11;
+        const double b00 = u.x * a00 - u.y * a10, b01 = u.x * a01 - u.y * a11;  // rows
+        const double b10 = u.y * a00 + u.x * a10, b11 = u.y * a01 + u.x * a11;
+        *x00 = v.x * b00 - v.y * b01;  // columns
+        *x01 = v.y * b00 + v.x * b01;
+        if (bk[t] != bl[t]) *x10 = v.x * b10 - v.y * b11;  // (k, k): the mirror image of x01
+        *x11 = v.y * b10 + v.x * b11;
       }
       __syncthreads();
     }
-    if (rotated == 0) break;
+    if (rotated == 0) {
+      ++sweep;
+      break;
+    }
   }
-  // sort eigenvalues descending (only the first n indices are real)
-  if (tid == 0) {
-    for (int i = 0; i < n; ++i) order[i] = i;
-    for (int i = 0; i < n; ++i)
-      for (int j = i + 1; j < n; ++j)
-        if (A[order[j] * ld + order[j]] > A[order[i] * ld + order[i]]) {
-          int t = order[i];
-          order[i] = order[j];
-          order[j] = t;
+  // eigenvalues descending (only the first n indices are real)
+  if (tid == 0) *sweeps = sweep;
+  auto key = [&](int j) {  // orders as the value, NaNs included
+    const long long b = __double_as_longlong(A[j * ld + j]);
+    return b < 0 ? ~(unsigned long long)b : (unsigned long long)b | 0x8000000000000000ull;
+  };
+  for (int j = tid; j < n; j += nt) {
+    const unsigned long long x = key(j);
+    int r = 0;
+    for (int i = 0; i < n; ++i) {
+      const unsigned long long y = key(i);
+      r += y > x || (y == x && i < j);
+    }
+    place[j] = r;
+    w_out[r] = scalbn(A[j * ld + j], e);
+  }
+}
+
+// Row blockIdx.x of V = I J_1 J_2 ..., columns at their places
+__global__ void __launch_bounds__(32) jacobi_vectors_kernel(const double2 *rot, const int *place, const int *sweeps,
+                                                            int n, double *V_out) {
+  __shared__ double v[kJacobiMax];
+  const int np = (n + 1) & ~1, half = np / 2, lane = threadIdx.x, row = blockIdx.x;
+  for (int j = lane; j < np; j += 32) v[j] = j == row ? 1.0 : 0.0;
+  __syncwarp();
+  const int steps = *sweeps * (np - 1);
+  constexpr int kPer = (kJacobiMax / 2 + 31) / 32, kAhead = 8;  // steps in flight
+  auto fetch = [&](int t, double2 (&r)[kPer]) {
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+      r[i] = t < steps && lane + 32 * i < half ? rot[(size_t)t * half + lane + 32 * i] : make_double2(1.0, 0.0);
+  };
+  double2 nx[kAhead][kPer];
+#pragma unroll
+  for (int a = 0; a < kAhead; ++a) fetch(a, nx[a]);
+  for (int t0 = 0, step = 0; t0 < steps; t0 += kAhead) {
+#pragma unroll
+    for (int a = 0; a < kAhead; ++a) {  // the steps past the last are identities
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const double2 r = nx[a][i];
+        if (lane + 32 * i < half && r.y != 0.0) {
+          int p, q;
+          jacobi_pair(lane + 32 * i, step, np, p, q);
+          const double x = v[p], y = v[q];
+          v[p] = r.x * x - r.y * y;
+          v[q] = r.y * x + r.x * y;
         }
+      }
+      fetch(t0 + kAhead + a, nx[a]);
+      __syncwarp();
+      step = step + 1 == np - 1 ? 0 : step + 1;
+    }
   }
-  __syncthreads();
-  for (int i = tid; i < n; i += nt) w_out[i] = A[order[i] * ld + order[i]];
-  for (int idx = tid; idx < n * n; idx += nt) {
-    int row = idx / n, k = idx % n;
-    V_out[idx] = V[row * ld + order[k]];
-  }
+  for (int j = lane; j < n; j += 32) V_out[(size_t)row * n + place[j]] = v[j];
 }
 
 // ------------------------------------------------------------- misc
@@ -783,9 +878,14 @@ void gemm(cudaStream_t st, int M, int N, int K, T alpha, const T *A, int lda, bo
       }
     }
   }
-  const int tm = cdiv(M, BM), tn = cdiv(N, BN);
+  const int nb = N <= 32 && !sym_upper ? 32 : 64;
+  const int tm = cdiv(M, BM), tn = cdiv(N, nb);
   long long tiles = sym_upper ? (long long)tm * (tm + 1) / 2 : (long long)tm * tn;
-  int splits = (int)std::max<long long>(1, std::min<long long>((296 + tiles - 1) / tiles, cdiv(K, 256)));
+  // K splits up to two CTAs per SM, each of at least 4 k blocks (8 where the
+  // partial sums to be added would be many): a block costs about 0.6 us whatever
+  // the tile, and the eigensolver's products of a few tiles and K = 250 or 3,876
+  // took 45 us with splits of at least 256
+  int splits = (int)std::max<long long>(1, std::min<long long>((296 + tiles - 1) / tiles, cdiv(K, K > 1024 ? 128 : 64)));
   int kchunk = (int)(cdiv(cdiv(K, splits), BK) * BK);
   splits = std::max(1, (int)cdiv(K, kchunk));
   const bool direct = splits == 1 && alpha == T(1) && beta == T(0) && !sym_upper;
@@ -794,9 +894,15 @@ void gemm(cudaStream_t st, int M, int N, int K, T alpha, const T *A, int lda, bo
   const int ldo = direct ? ldc : N;
   const size_t stride = (size_t)M * N;
   dim3 grid(tn, tm, splits);
-#define SPB_GEMM_LAUNCH(TA, TB, KS)                                                            \
-  gemm_tile_kernel<T, TA, TB, KS><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, kscale, out, \
-                                                        ldo, kchunk, sym_upper ? 1 : 0, stride)
+#define SPB_GEMM_LAUNCH(TA, TB, KS)                                                                          \
+  do {                                                                                                       \
+    if (nb == 32)                                                                                            \
+      gemm_tile_kernel<T, 32, TA, TB, KS><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, kscale, out, ldo,   \
+                                                                kchunk, 0, stride);                          \
+    else                                                                                                     \
+      gemm_tile_kernel<T, 64, TA, TB, KS><<<grid, 256, 0, st>>>(M, N, K, A, lda, B, ldb, kscale, out, ldo,   \
+                                                                kchunk, sym_upper ? 1 : 0, stride);          \
+  } while (0)
   const bool ks = kscale != nullptr;
   if (transA && transB) { if (ks) SPB_GEMM_LAUNCH(true, true, true); else SPB_GEMM_LAUNCH(true, true, false); }
   else if (transA) { if (ks) SPB_GEMM_LAUNCH(true, false, true); else SPB_GEMM_LAUNCH(true, false, false); }
@@ -917,10 +1023,17 @@ static void project_out(cudaStream_t st, const double *Q, int ldq, int width, do
 
 void jacobi_eig(cudaStream_t st, const double *S, int n, double *w, double *V) {
   if (n > kJacobiMax) fail(SYMPROP_ERR_SIZE, "jacobi_eig: n=%d > %d", n, kJacobiMax);
-  int np = (n + 1) & ~1;
-  size_t smem = 2 * sizeof(double) * np * (np + 1);
+  const int np = (n + 1) & ~1, half = np / 2, blocks = half * (half + 1) / 2;
+  const size_t smem = sizeof(double) * np * (np + 1);
+  Scratch rot(sizeof(double2) * (size_t)kJacobiSweeps * std::max(np - 1, 1) * half, st),
+      meta(sizeof(int) * (n + 1), st);
+  int *place = meta.as<int>(), *sweeps = place + n;
   SPB_CUDA(cudaFuncSetAttribute(jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  jacobi_kernel<<<1, 1024, smem, st>>>(S, n, w, V);
+  // one block of A per thread where 1024 threads can, else two
+  const int threads = std::min(1024, std::max(64, (int)cdiv(blocks > 1024 ? cdiv(blocks, 2) : blocks, 32) * 32));
+  jacobi_kernel<<<1, threads, smem, st>>>(S, n, w, rot.as<double2>(), place, sweeps);
+  SPB_LAUNCH_CHECK();
+  jacobi_vectors_kernel<<<n, 32, 0, st>>>(rot.as<double2>(), place, sweeps, n, V);
   SPB_LAUNCH_CHECK();
 }
 
