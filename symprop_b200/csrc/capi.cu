@@ -226,13 +226,13 @@ int symprop_symsyrk_device(const float *dA, const float *dscale, double *dC, uin
     require(dA && dscale && dC, "null argument");
     require(ncoeff > 0 && I1 > 0 && ncoeff < (1ull << 31) && I1 < (1ull << 31), "bad sizes");
     cudaStream_t st = (cudaStream_t)stream;
-    DBuf<char> ws(gram::split_bytes((int)I1, (int)ncoeff)), scr(gram::gram_rows_scratch_bytes((int)I1, (int)ncoeff));
-    DBuf<int> err(1);
+    PoolBuf ws(gram::split_bytes((int)I1, (int)ncoeff), st), scr(gram::gram_rows_scratch_bytes((int)I1, (int)ncoeff), st);
+    PoolBuf err(sizeof(int), st);
     SPB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
     const gram::Split z = gram::split_view(ws.p, (int)I1, (int)ncoeff);
     gram::split(st, dA, dscale, z);
-    gram::gram_rows(st, z, dC, scr.p, err.p);
-    check_tc_err(st, err.p);
+    gram::gram_rows(st, z, dC, scr.p, err.as<int>());
+    check_tc_err(st, err.as<int>());
   });
 }
 
@@ -243,17 +243,17 @@ int symprop_symgemm_device(const float *dA, const double *dB, const double *dsca
     require(ncoeff > 0 && I1 > 0 && I2 > 0 && ncoeff < (1ull << 31) && I1 < (1ull << 31) && I2 < (1ull << 20),
             "bad sizes");
     cudaStream_t st = (cudaStream_t)stream;
-    DBuf<char> ws(gram::split_bytes((int)I1, (int)ncoeff)), scr(gram::times_scratch_bytes((int)I1, (int)ncoeff));
-    DBuf<float> sc((size_t)ncoeff);
-    DBuf<int> err(1);
+    PoolBuf ws(gram::split_bytes((int)I1, (int)ncoeff), st), scr(gram::times_scratch_bytes((int)I1, (int)ncoeff), st);
+    PoolBuf sc(sizeof(float) * (size_t)ncoeff, st);
+    PoolBuf err(sizeof(int), st);
     SPB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
-    dense::convert<double, float>(st, dscale, sc.p, (size_t)ncoeff);
+    dense::convert<double, float>(st, dscale, sc.as<float>(), (size_t)ncoeff);
     const gram::Split z = gram::split_view(ws.p, (int)I1, (int)ncoeff);
-    gram::split(st, dA, sc.p, z);
+    gram::split(st, dA, sc.as<float>(), z);
     for (uint64_t q0 = 0; q0 < I2; q0 += gram::kPanelRows)
       gram::times(st, z, dB + q0 * ncoeff, (int)std::min<uint64_t>(gram::kPanelRows, I2 - q0), (size_t)ncoeff, 1,
-                  dscale, dC + q0, (size_t)I2, scr.p, err.p);
-    check_tc_err(st, err.p);
+                  dscale, dC + q0, (size_t)I2, scr.p, err.as<int>());
+    check_tc_err(st, err.as<int>());
   });
 }
 
@@ -269,11 +269,11 @@ int symprop_gram_device(const void *dY, uint64_t n, uint32_t m, const void *dsca
                           (int)m, nullptr, true);
       dense::scale_sym(st, dG, (int)m, sd);
     } else if (precision == SYMPROP_FP32) {
-      DBuf<char> ws(gram::workspace_bytes((int)n, (int)m));
-      DBuf<int> err(1);
+      PoolBuf ws(gram::workspace_bytes((int)n, (int)m), st);
+      PoolBuf err(sizeof(int), st);
       SPB_CUDA(cudaMemsetAsync(err.p, 0, sizeof(int), st));
       gram::gram_split_bf16(st, (const float *)dY, (int)n, (int)m, (const float *)dscale, dG, ws.p,
-                            err.p);
+                            err.as<int>());
       int h = 0;
       SPB_CUDA(cudaMemcpyAsync(&h, err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
       SPB_CUDA(cudaStreamSynchronize(st));

@@ -126,6 +126,29 @@ template <class T> struct DBuf {
 };
 
 
+// Workspace of one call on `st` from that pool, so that a repeated call waits for
+// no allocation (an FP32 Gram of 50,000 x 2,002: 1.8 to 11.8 ms with cudaMalloc
+// and cudaFree per call).  Larger ones than kPoolMax are not kept: they are
+// allocated and freed by themselves.
+struct PoolBuf {
+  static constexpr size_t kPoolMax = 9ull << 29;  // 4.5 GB
+  void *p = nullptr;
+  cudaStream_t st;
+  bool pooled = true;
+  PoolBuf(size_t bytes, cudaStream_t s) : st(s), pooled(bytes <= kPoolMax) {
+    if (!bytes) return;
+    if (pooled) SPB_CUDA(cudaMallocFromPoolAsync(&p, bytes, device_pool(), st));
+    else SPB_CUDA(cudaMalloc(&p, bytes));
+  }
+  PoolBuf(const PoolBuf &) = delete;
+  PoolBuf &operator=(const PoolBuf &) = delete;
+  ~PoolBuf() {
+    if (p && pooled) cudaFreeAsync(p, st);
+    else if (p) cudaFree(p);
+  }
+  template <class T> T *as() const { return reinterpret_cast<T *>(p); }
+};
+
 // ------------------------------------------------------- packed indexing
 
 inline uint64_t binom(uint64_t n, uint64_t k) {

@@ -802,19 +802,7 @@ __global__ void residual_kernel(const double *SX, const double *X, int s, int ld
   if (threadIdx.x == 0) res[i] = sqrt(red[0]);
 }
 
-cudaMemPool_t scratch_pool() { return device_pool(); }
-
-struct Scratch {
-  void *p = nullptr;
-  cudaStream_t st = 0;
-  Scratch(size_t bytes, cudaStream_t s) : st(s) {
-    if (bytes) SPB_CUDA(cudaMallocFromPoolAsync(&p, bytes, scratch_pool(), st));
-  }
-  ~Scratch() {
-    if (p) cudaFreeAsync(p, st);
-  }
-  template <class T> T *as() { return reinterpret_cast<T *>(p); }
-};
+using Scratch = PoolBuf;
 
 // Partial core products P[chunk][q][j] = sum_{i in chunk} U[i][q0 + q] Y[i][j]
 // over FP32 Y (n x m, read once, coalesced along j) and FP64 U (n x r): one
