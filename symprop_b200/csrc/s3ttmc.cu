@@ -439,7 +439,8 @@ uint32_t s3ttmc_launch_count(const TensorState &t, uint32_t R, bool packed) {
   if (t.order <= 2) return packed ? 1 : 1;
   const bool chain = (s3ttmc_schedule() == kScheduleAuto || s3ttmc_schedule() == kScheduleChain) &&
                      chain_supported(t, R);
-  const uint32_t nsplit = chain && t.chain ? t.chain->nsplit : t.nsplit;
+  const ChainItems *items = chain ? built_chain_items(t, R) : nullptr;
+  const uint32_t nsplit = items ? items->nsplit : t.nsplit;
   uint32_t n = 1;                 // S3TTMc kernel
   if (s3ttmc_schedule() == kScheduleAuto && split_supported(t.order, R)) {
     ItemSet all;
@@ -448,7 +449,7 @@ uint32_t s3ttmc_launch_count(const TensorState &t, uint32_t R, bool packed) {
     const uint32_t nh = split_heavy(R, all);
     if (nh && nh < t.nchunks) n += 1;  // warp kernel of the light rows
   }
-  if (chain && t.chain && t.chain->nlight) n += 1;  // warp kernel of the light rows
+  if (items && items->nlight) n += 1;  // warp kernel of the light rows
   if (nsplit) n += 1;             // combine kernel
   if (!packed) n += 1;            // unpack kernel
   return n;
@@ -671,7 +672,7 @@ static void s3ttmc_reserve(TensorState &t, uint32_t R, bool packed, int precisio
   const uint64_t m = symsize(R, t.order - 1);
   if (!packed && t.order > 2) t.scratch.ensure((size_t)t.dim * m * es);
   uint32_t slots = t.nslots;
-  if (use_chain(t, R)) slots = std::max(slots, chain_data(t).nslots);
+  if (use_chain(t, R)) slots = std::max(slots, chain_items(t, R).nslots);
   if (slots) t.partials.ensure((size_t)slots * m);
 }
 
@@ -685,7 +686,7 @@ void s3ttmc_run(TensorState &t, const void *dU, uint32_t R, bool packed, void *d
   s3ttmc_reserve(t, R, packed, precision);
   ItemSet all;
   if (use_chain(t, R)) {
-    const ChainData &cd = chain_data(t);
+    const ChainItems &cd = chain_items(t, R);
     all.chunks = cd.chunks.p;
     all.nchunks = cd.nchunks;
     all.split = cd.split.p;
@@ -753,7 +754,7 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
   t.io_U.ensure(ubytes);
   t.io_Y.ensure(ybytes);
   const bool chain = use_chain(t, R);
-  const RowBands &bd = chain ? chain_bands(t, host_band_count(ybytes)) : row_bands(t, host_band_count(ybytes));
+  const RowBands &bd = chain ? chain_bands(t, R, host_band_count(ybytes)) : row_bands(t, host_band_count(ybytes));
 
   // SPB_TRACE_HOST=1 prints when each band's compute and copy ended
   const bool trace = std::getenv("SPB_TRACE_HOST") != nullptr;
@@ -791,7 +792,7 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
     band.row0 = bd.row0[k];
     band.rows = bd.row0[k + 1] - bd.row0[k];
     band.chain = chain;
-    band.nslots = chain ? t.chain->nslots : t.nslots;
+    band.nslots = chain ? chain_items(t, R).nslots : t.nslots;
     if (!chain) band.nheavy = bd.nheavy[k];
     if (chain) {
       band.light = bd.light.p + bd.light0[k];

@@ -1,5 +1,6 @@
 // S3TTMc, pivot-chain schedule (order 4 / R <= 16): the owners of a row are
-// contracted pivot by pivot instead of leaf by leaf.
+// contracted pivot by pivot instead of leaf by leaf.  (R <= 8 runs the warp
+// kernel of s3ttmc_chain8.cu on the data that is built here.)
 //
 // The reference's leaf tensor (SymOuterProd recursion,
 // include/detail/dense/symtensor.hpp:24-39, src/compressed_dtree.cpp:421-518)
@@ -39,6 +40,7 @@
 
 #include "check.cuh"
 #include "s3ttmc_chain.cuh"
+#include "s3ttmc_chain8.cuh"
 
 namespace spb {
 namespace {
@@ -925,31 +927,48 @@ ChainData &chain_data(TensorState &t) {
     chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S.p, rows_b.p, nown, t.sstride, L, cd->flags.p);
     SPB_LAUNCH_CHECK();
   }
-  // work items: the rows' owner ranges are unchanged (the sort keeps rows);
-  // light rows one item each, heavy rows cut into items of at most co owners
-  const uint64_t heavy_owners = heavy_owner_count(t);
-  const uint64_t target_items = 148ull * 4ull * 8ull;
-  uint64_t co = (heavy_owners + target_items - 1) / target_items;
-  co = std::min<uint64_t>(std::max<uint64_t>(co, 256), 1024);
-  cd->chunk_owners = (uint32_t)co;
-  std::vector<Chunk> ch, lt;
-  std::vector<SplitRow> sp;
-  cd->nslots = cut_chain_rows(t, co, 0, t.dim, ch, sp, lt);
-  sort_heaviest_first(ch, 0, ch.size(), co);
-  sort_heaviest_first(lt, 0, lt.size(), kChainLight);
-  cd->nchunks = (uint32_t)ch.size();
-  cd->nsplit = (uint32_t)sp.size();
-  cd->nlight = (uint32_t)lt.size();
-  upload(cd->chunks, ch);
-  upload(cd->split, sp);
-  upload(cd->light, lt);
   SPB_CUDA(cudaDeviceSynchronize());
   t.chain = cd;
   return *cd;
 }
 
-const RowBands &chain_bands(TensorState &t, uint32_t nb) {
+// Work items: light rows one item each, heavy rows cut into items of at most co
+// owners: 32 an SM (eight waves of the resident CTAs, two of the warps), within
+// [256, 1024] owners for the CTA kernels and [64, 1024] for the warp kernel.  The warp kernel takes an
+// item's owners 32 at a time, so that on a small tensor its time is one item's:
+// 1,000 nodes, 20,000 entries, R = 6 in FP32: 41 us with items of 256, 27 us
+// with 64.  The
+// CTA kernels lose with smaller items (R = 16, 128 instead of 256: 0.192 -> 0.215
+// ms on 10,000 nodes, 200,000 entries), their cost per item being larger.
+ChainItems &chain_items(TensorState &t, uint32_t R) {
   ChainData &cd = chain_data(t);
+  const bool warp = chain8_supported(t, R);
+  std::unique_ptr<ChainItems> &slot = cd.items[warp];
+  if (slot) return *slot;
+  auto it = std::make_unique<ChainItems>();
+  const uint64_t target_items = 148ull * 32ull;
+  const uint64_t co = (heavy_owner_count(t) + target_items - 1) / target_items;
+  it->chunk_owners = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(co, warp ? 64 : 256), 1024);
+  std::vector<Chunk> ch, lt;
+  std::vector<SplitRow> sp;
+  it->nslots = cut_chain_rows(t, it->chunk_owners, 0, t.dim, ch, sp, lt);
+  sort_heaviest_first(ch, 0, ch.size(), it->chunk_owners);
+  sort_heaviest_first(lt, 0, lt.size(), kChainLight);
+  it->nchunks = (uint32_t)ch.size();
+  it->nsplit = (uint32_t)sp.size();
+  it->nlight = (uint32_t)lt.size();
+  upload(it->chunks, ch);
+  upload(it->split, sp);
+  upload(it->light, lt);
+  return *(slot = std::move(it));
+}
+
+const ChainItems *built_chain_items(const TensorState &t, uint32_t R) {
+  return t.chain ? t.chain->items[chain8_supported(t, R)].get() : nullptr;
+}
+
+const RowBands &chain_bands(TensorState &t, uint32_t R, uint32_t nb) {
+  ChainItems &cd = chain_items(t, R);
   nb = std::max<uint32_t>(1, std::min<uint32_t>(nb, std::max<uint32_t>(t.dim, 1)));
   auto found = cd.bands.find(nb);
   if (found != cd.bands.end()) return *found->second;
@@ -1070,7 +1089,7 @@ void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &ite
   p.quad = tb.quad;
   p.nown = t.nown;
   p.nrows = t.dim;
-  p.nslots = cd.nslots;
+  p.nslots = items.nslots;
   if (precision == SYMPROP_FP64) {
     const size_t smem = sizeof(Smem5<double>);
     SPB_CUDA(cudaFuncSetAttribute(s3ttmc_chain5_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1095,6 +1114,10 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
     chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
     return;
   }
+  if (chain8_supported(t, R)) {  // one 8-wide tile: one warp per item (both sides measured there)
+    chain8_launch(t, cd, items, dU, R, dYpacked, precision, st);
+    return;
+  }
   ChainParams p;
   p.chunks = items.chunks;
   p.nchunks = items.nchunks;
@@ -1111,7 +1134,7 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
   p.trip = triples(R);
   p.nown = t.nown;
   p.nrows = t.dim;
-  p.nslots = cd.nslots;
+  p.nslots = items.nslots;
   if (precision == SYMPROP_FP64) {
     const size_t smem = sizeof(Smem<double>);
     SPB_CUDA(cudaFuncSetAttribute(s3ttmc_chain_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

@@ -5,13 +5,8 @@
 
 namespace spb {
 
-// Owners re-sorted for the chain schedule, built on first use.
-struct ChainData {
-  uint32_t L = 0;                 // leaf size (order - 1)
-  DBuf<uint32_t> S;               // nown x sstride leaf ids, highest-degree first
-  DBuf<double> c64;               // owner coefficients in chain order
-  DBuf<float> c32;
-  DBuf<uint8_t> flags;            // bit k: the owner starts a new prefix of k+1 pivots
+// Work items of the chain schedule, all rows and by bands.
+struct ChainItems {
   uint32_t chunk_owners = 0;
   uint32_t nchunks = 0, nsplit = 0, nslots = 0;
   DBuf<Chunk> chunks;             // work items of the heavy rows, heaviest first
@@ -19,6 +14,18 @@ struct ChainData {
   uint32_t nlight = 0;            // rows of at most kChainLight owners, one item
   DBuf<Chunk> light;              // each, for the warp-per-row kernel, heaviest first
   std::map<uint32_t, std::unique_ptr<RowBands>> bands;  // by band count
+};
+
+// Owners re-sorted for the chain schedule, built on first use.
+struct ChainData {
+  uint32_t L = 0;                 // leaf size (order - 1)
+  DBuf<uint32_t> S;               // nown x sstride leaf ids, highest-degree first
+  DBuf<double> c64;               // owner coefficients in chain order
+  DBuf<float> c32;
+  DBuf<uint8_t> flags;            // bit k: the owner starts a new prefix of k+1 pivots
+  // items, by kernel: of 256 owners at least (a CTA each), of 64 at least (a warp
+  // each: order 4, R <= 8)
+  std::unique_ptr<ChainItems> items[2];
 };
 
 // Order 4: rows with at most this many owners share few pivots; the chain
@@ -31,8 +38,10 @@ uint64_t chain_light_max(const TensorState &t);
 bool chain_supported(const TensorState &t, uint32_t R);
 // The chain data of t (built on the first call).
 ChainData &chain_data(TensorState &t);
-// The chain work items in nb row bands (built on first use).
-const RowBands &chain_bands(TensorState &t, uint32_t nb);
+// The work items of rank R (built on first use), and in nb row bands.
+ChainItems &chain_items(TensorState &t, uint32_t R);
+const ChainItems *built_chain_items(const TensorState &t, uint32_t R);  // null before the first use
+const RowBands &chain_bands(TensorState &t, uint32_t R, uint32_t nb);
 // One pass over chain work items: packed Y rows, partial rows for split rows.
 void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
                   void *dYpacked, int precision, cudaStream_t st);
