@@ -136,7 +136,8 @@ int symprop_s3ttmc(const symprop_tensor *t, const void *U, uint32_t R,
 int symprop_s3ttmc_device(const symprop_tensor *t, const void *dU, uint32_t R,
                           int packed, void *dY, int precision, void *stream);
 /* Selects the S3TTMc schedule for the whole process: 0 automatic (default:
- * the pivot chain where it applies (order 4 at R <= 8: its warp kernel), else the split-leaf product (order 6,
+ * the pivot chain where it applies (order 4 at R <= 8: its warp kernel;
+ * order 5: its group kernel where that is the faster one), else the split-leaf product (order 6,
  * R <= 10), else warp-per-owner where the packed
  * output fits one warp's registers, else CTA register-tiled, else the
  * per-owner rows kernel), 1 rows kernel, 2 CTA register-tiled only,

@@ -672,7 +672,7 @@ static void s3ttmc_reserve(TensorState &t, uint32_t R, bool packed, int precisio
   const uint64_t m = symsize(R, t.order - 1);
   if (!packed && t.order > 2) t.scratch.ensure((size_t)t.dim * m * es);
   uint32_t slots = t.nslots;
-  if (use_chain(t, R)) slots = std::max(slots, chain_items(t, R).nslots);
+  if (use_chain(t, R)) slots = std::max(slots, chain_items(t, R, precision).nslots);
   if (slots) t.partials.ensure((size_t)slots * m);
 }
 
@@ -686,7 +686,8 @@ void s3ttmc_run(TensorState &t, const void *dU, uint32_t R, bool packed, void *d
   s3ttmc_reserve(t, R, packed, precision);
   ItemSet all;
   if (use_chain(t, R)) {
-    const ChainItems &cd = chain_items(t, R);
+    const ChainItems &cd = chain_items(t, R, precision);
+    all.groups = cd.groups;
     all.chunks = cd.chunks.p;
     all.nchunks = cd.nchunks;
     all.split = cd.split.p;
@@ -754,7 +755,7 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
   t.io_U.ensure(ubytes);
   t.io_Y.ensure(ybytes);
   const bool chain = use_chain(t, R);
-  const RowBands &bd = chain ? chain_bands(t, R, host_band_count(ybytes)) : row_bands(t, host_band_count(ybytes));
+  const RowBands &bd = chain ? chain_bands(t, R, precision, host_band_count(ybytes)) : row_bands(t, host_band_count(ybytes));
 
   // SPB_TRACE_HOST=1 prints when each band's compute and copy ended
   const bool trace = std::getenv("SPB_TRACE_HOST") != nullptr;
@@ -792,7 +793,8 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
     band.row0 = bd.row0[k];
     band.rows = bd.row0[k + 1] - bd.row0[k];
     band.chain = chain;
-    band.nslots = chain ? chain_items(t, R).nslots : t.nslots;
+    band.nslots = chain ? chain_items(t, R, precision).nslots : t.nslots;
+    band.groups = chain && chain_items(t, R, precision).groups;
     if (!chain) band.nheavy = bd.nheavy[k];
     if (chain) {
       band.light = bd.light.p + bd.light0[k];

@@ -437,6 +437,8 @@ __global__ void __launch_bounds__(kThreads, 4) s3ttmc_chain_kernel(const ChainPa
 
 // ----------------------------------------------------- order 5 (L = 4)
 //
+// (Where s3ttmc_chain5.cu is not the faster one: chain5_pays.)
+//
 // Leaf S = {s_1, s_2, s_3, s_4} in pivot order.  With the owners of a row
 // sorted by (s_1, s_2):
 //   T3_h = sum over the owners of h = (s_1, s_2) of c * K({s_3, s_4})  (order 2, m2)
@@ -849,6 +851,21 @@ uint32_t cut_chain_rows(const TensorState &t, uint64_t co, uint32_t r0, uint32_t
   return slot;
 }
 
+// Sorts items ch[b, e) (ranges of owners, in row order from item b on) by owners,
+// heaviest first.  Group kernel: they become (item number, number of sub-groups)
+// ranges.
+void sort_chain_items(const ChainData &cd, const ChainItems &it, std::vector<Chunk> &ch, size_t b, size_t e) {
+  if (it.groups)  // carry the item's number through the sort
+    for (size_t i = b; i < e; ++i) {
+      const uint64_t k = ch[i].oe - ch[i].ob;
+      ch[i].ob = i;
+      ch[i].oe = i + k;
+    }
+  sort_heaviest_first(ch, b, e, it.chunk_owners);
+  if (it.groups)
+    for (size_t i = b; i < e; ++i) ch[i].oe = ch[i].ob + cd.groups->sub[ch[i].ob];
+}
+
 }  // namespace
 
 bool chain_supported(const TensorState &t, uint32_t R) {
@@ -940,19 +957,30 @@ ChainData &chain_data(TensorState &t) {
 // with 64.  The
 // CTA kernels lose with smaller items (R = 16, 128 instead of 256: 0.192 -> 0.215
 // ms on 10,000 nodes, 200,000 entries), their cost per item being larger.
-ChainItems &chain_items(TensorState &t, uint32_t R) {
+ChainItems &chain_items(TensorState &t, uint32_t R, int precision) {
   ChainData &cd = chain_data(t);
   const bool warp = chain8_supported(t, R);
-  std::unique_ptr<ChainItems> &slot = cd.items[warp];
+  const bool groups = !cd.no_groups && chain5_pays(t, R, precision);
+  std::unique_ptr<ChainItems> &slot = cd.items[warp || groups];
   if (slot) return *slot;
   auto it = std::make_unique<ChainItems>();
   const uint64_t target_items = 148ull * 32ull;
   const uint64_t co = (heavy_owner_count(t) + target_items - 1) / target_items;
   it->chunk_owners = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(co, warp ? 64 : 256), 1024);
+  it->groups = groups;
   std::vector<Chunk> ch, lt;
   std::vector<SplitRow> sp;
   it->nslots = cut_chain_rows(t, it->chunk_owners, 0, t.dim, ch, sp, lt);
-  sort_heaviest_first(ch, 0, ch.size(), it->chunk_owners);
+  if (groups && !cd.groups) {
+    try {
+      cd.groups = chain5_build(t, cd, ch);
+    } catch (const Error &e) {  // no memory for a second copy of the owners
+      if (e.code != SYMPROP_ERR_OOM) throw;
+      cd.no_groups = true;
+      return chain_items(t, R, precision);
+    }
+  }
+  sort_chain_items(cd, *it, ch, 0, ch.size());
   sort_heaviest_first(lt, 0, lt.size(), kChainLight);
   it->nchunks = (uint32_t)ch.size();
   it->nsplit = (uint32_t)sp.size();
@@ -963,12 +991,16 @@ ChainItems &chain_items(TensorState &t, uint32_t R) {
   return *(slot = std::move(it));
 }
 
+// (the split rows and light rows of the two order-5 kernels are the same)
 const ChainItems *built_chain_items(const TensorState &t, uint32_t R) {
-  return t.chain ? t.chain->items[chain8_supported(t, R)].get() : nullptr;
+  if (!t.chain) return nullptr;
+  const auto &items = t.chain->items;
+  if (t.order == 5) return items[0] ? items[0].get() : items[1].get();
+  return items[chain8_supported(t, R)].get();
 }
 
-const RowBands &chain_bands(TensorState &t, uint32_t R, uint32_t nb) {
-  ChainItems &cd = chain_items(t, R);
+const RowBands &chain_bands(TensorState &t, uint32_t R, int precision, uint32_t nb) {
+  ChainItems &cd = chain_items(t, R, precision);
   nb = std::max<uint32_t>(1, std::min<uint32_t>(nb, std::max<uint32_t>(t.dim, 1)));
   auto found = cd.bands.find(nb);
   if (found != cd.bands.end()) return *found->second;
@@ -993,7 +1025,7 @@ const RowBands &chain_bands(TensorState &t, uint32_t R, uint32_t nb) {
     b->light0[k] = before(lt);
   }
   for (uint32_t k = 0; k < nb; ++k) {
-    sort_heaviest_first(ch, b->chunk0[k], b->chunk0[k + 1], cd.chunk_owners);
+    sort_chain_items(*t.chain, cd, ch, b->chunk0[k], b->chunk0[k + 1]);
     sort_heaviest_first(lt, b->light0[k], b->light0[k + 1], kChainLight);
   }
   upload(b->chunks, ch);
@@ -1069,7 +1101,7 @@ const Order5Tables &order5_tables(uint32_t R) {
   return tb;
 }
 
-void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
+void chain5_rows_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
                    void *dYpacked, int precision, cudaStream_t st) {
   const Order5Tables &tb = order5_tables(R);
   Chain5Params p;
@@ -1111,7 +1143,8 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
   if (!chain_supported(t, R)) fail(SYMPROP_ERR_SIZE, "chain S3TTMc does not support order %u rank %u", t.order, R);
   if (!items.nchunks) return;
   if (t.order == 5) {
-    chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
+    if (items.groups) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
+    else chain5_rows_launch(t, cd, items, dU, R, dYpacked, precision, st);
     return;
   }
   if (chain8_supported(t, R)) {  // one 8-wide tile: one warp per item (both sides measured there)

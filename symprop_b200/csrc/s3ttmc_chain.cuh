@@ -14,6 +14,16 @@ struct ChainItems {
   uint32_t nlight = 0;            // rows of at most kChainLight owners, one item
   DBuf<Chunk> light;              // each, for the warp-per-row kernel, heaviest first
   std::map<uint32_t, std::unique_ptr<RowBands>> bands;  // by band count
+  bool groups = false;            // order 5: items of s3ttmc_chain5.cu
+};
+
+// Order 5: the owners of every item in the order the building warps of
+// s3ttmc_chain5.cu take them.  Built on first use of a rank it covers.
+struct ChainGroups {
+  DBuf<uint32_t> S;               // nown x 4 leaf ids in pivot order; bit 31 of s_1: ends its sub-group
+  DBuf<double> c;                 // owner coefficients
+  DBuf<uint32_t> first;           // per item in row order: the first owner of each warp, the item's end
+  std::vector<uint32_t> sub;      // per item: its sub-groups
 };
 
 // Owners re-sorted for the chain schedule, built on first use.
@@ -23,8 +33,10 @@ struct ChainData {
   DBuf<double> c64;               // owner coefficients in chain order
   DBuf<float> c32;
   DBuf<uint8_t> flags;            // bit k: the owner starts a new prefix of k+1 pivots
-  // items, by kernel: of 256 owners at least (a CTA each), of 64 at least (a warp
-  // each: order 4, R <= 8)
+  std::unique_ptr<ChainGroups> groups;
+  bool no_groups = false;         // no memory for them: the CTA kernel runs instead
+  // items, by kernel: the CTA kernels; the warp kernel (order 4, R <= 8) or the
+  // group kernel (order 5)
   std::unique_ptr<ChainItems> items[2];
 };
 
@@ -38,12 +50,22 @@ uint64_t chain_light_max(const TensorState &t);
 bool chain_supported(const TensorState &t, uint32_t R);
 // The chain data of t (built on the first call).
 ChainData &chain_data(TensorState &t);
-// The work items of rank R (built on first use), and in nb row bands.
-ChainItems &chain_items(TensorState &t, uint32_t R);
+// The work items of a rank and precision (built on first use), and in nb row bands.
+ChainItems &chain_items(TensorState &t, uint32_t R, int precision);
 const ChainItems *built_chain_items(const TensorState &t, uint32_t R);  // null before the first use
-const RowBands &chain_bands(TensorState &t, uint32_t R, uint32_t nb);
+const RowBands &chain_bands(TensorState &t, uint32_t R, int precision, uint32_t nb);
 // One pass over chain work items: packed Y rows, partial rows for split rows.
 void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
                   void *dYpacked, int precision, cudaStream_t st);
+
+
+// s3ttmc_chain5.cu (order 5): whether the group kernel is the faster one here;
+// the owners of items (ranges in row order of the owners in pivot order), dealt to
+// its warps; one pass over items whose ob is the item's number in row order and
+// whose oe - ob is its number of sub-groups.
+bool chain5_pays(const TensorState &t, uint32_t R, int precision);
+std::unique_ptr<ChainGroups> chain5_build(const TensorState &t, const ChainData &cd, const std::vector<Chunk> &items);
+void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
+                   void *dYpacked, int precision, cudaStream_t st);
 
 }  // namespace spb

@@ -33,8 +33,8 @@
 #include <map>
 #include <mutex>
 
-#include "check.cuh"
 #include "s3ttmc_chain8.cuh"
+#include "s3ttmc_mma.cuh"
 
 namespace spb {
 namespace {
@@ -62,13 +62,6 @@ struct Params {
   uint64_t nown;
   uint32_t nrows, nslots;
 };
-
-// c (8 x 8, rows r8, columns 2 kq + {0, 1}) += a (8 x 4: row r8, column kq) * b (4 x 8: row kq, column r8)
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
 
 __device__ __forceinline__ uint32_t shared_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

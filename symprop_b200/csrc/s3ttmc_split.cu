@@ -40,6 +40,7 @@
 #include <type_traits>
 
 #include "check.cuh"
+#include "s3ttmc_mma.cuh"
 #include "s3ttmc_split.cuh"
 
 namespace spb {
@@ -84,24 +85,11 @@ struct SplitParams {
   double *partials;
   uint32_t m, npair, nelem;
   const uint32_t *pairs, *elems, *sym;
-  uint64_t nown;
+  uint64_t nentries;  // owners
   uint32_t nrows, nslots;
 };
 
 enum { kBarFull = 1, kBarEmpty = kBarFull + kStages, kBarM = kBarEmpty + kStages, kBarMFree };
-
-template <int THREADS> __device__ __forceinline__ void bar_sync(int id) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
-}
-template <int THREADS> __device__ __forceinline__ void bar_arrive(int id) {
-  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(THREADS) : "memory");
-}
-
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
-               : "d"(a), "d"(b));
-}
 
 // Three shared values: one 16-byte load of a group of four (FP32), three
 // 8-byte loads (FP64: groups of three fall on different banks, 16-byte loads
@@ -119,55 +107,6 @@ __device__ __forceinline__ void store3(double *p, double a, double b, double c) 
 // A staged leaf: RZ groups (U[s_1][x], U[s_2][x], U[s_3][x]), then RZ groups
 // (U[s_4][x], c U[s_5][x])
 template <typename T, int RZ> constexpr int kLeaf = RZ * (kG3<T> + 2);
-
-// The CTA's batches in order: the owners of items blockIdx.x, blockIdx.x +
-// gridDim.x, ..., 16 at a time.  Both roles walk the same sequence.
-struct Walk {
-  uint32_t item = 0, row = 0, slot = 0, o = 0, oe = 0;
-  bool first = false;  // the item's first batch
-  Chunk ahead{};       // the item to be opened next, loaded an item early
-  __device__ __forceinline__ void start(const SplitParams &p) {
-    item = blockIdx.x;
-    if (item < p.nchunks) ahead = p.chunks[item];
-  }
-  __device__ __forceinline__ bool valid(const SplitParams &p) const { return item < p.nchunks; }
-  __device__ __forceinline__ int count() const { return (int)min((uint32_t)kK, oe - o); }
-  __device__ __forceinline__ bool last() const { return oe - o <= (uint32_t)kK; }
-  // opens the first item with owners at or after `item`; empty(row, slot)
-  // is called for each one without
-  template <class Empty> __device__ __forceinline__ void open(const SplitParams &p, Empty &&empty) {
-    for (; item < p.nchunks; item += gridDim.x) {
-      const Chunk ch = ahead;
-      if (item + gridDim.x < p.nchunks) ahead = p.chunks[item + gridDim.x];
-      if (!SPB_BOUND(ch.ob <= ch.oe && ch.oe <= p.nown && ch.row < p.nrows &&
-                         (ch.slot == kDirect || ch.slot < p.nslots),
-                     501, item))
-        continue;
-      row = ch.row;
-      slot = ch.slot;
-      o = (uint32_t)ch.ob;
-      oe = (uint32_t)ch.oe;
-      first = true;
-      if (o < oe) return;
-      empty(row, slot);
-    }
-  }
-  template <class Empty> __device__ __forceinline__ void next(const SplitParams &p, Empty &&empty) {
-    if (!last()) {
-      o += kK;
-      first = false;
-    } else {
-      item += gridDim.x;
-      open(p, empty);
-    }
-  }
-};
-
-template <typename T>
-__device__ __forceinline__ void put(const SplitParams &p, uint32_t row, uint32_t slot, uint32_t e, double y) {
-  if (slot == kDirect) reinterpret_cast<T *>(p.Y)[(uint64_t)row * p.m + e] = (T)y;
-  else p.partials[(uint64_t)slot * p.m + e] = y;
-}
 
 template <int RZ, int BW, typename T> constexpr size_t split_smem(bool sym_shared, uint32_t m) {
   using G = Geo<RZ>;
@@ -205,7 +144,7 @@ __global__ void __launch_bounds__(kMul + 32 * BW, CTAS) s3ttmc_split_kernel(cons
 #pragma unroll
       for (int j = 0; j < G::NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
     auto none = [](uint32_t, uint32_t) {};
-    Walk w;
+    Walk<kK> w;
     w.start(p);
     w.open(p, none);
     bool m_used = false;
@@ -301,7 +240,7 @@ __global__ void __launch_bounds__(kMul + 32 * BW, CTAS) s3ttmc_split_kernel(cons
                           : -1;
   }
   const int own_l = lane / kL, place_l = lane - own_l * kL;
-  auto load_ids = [&](const Walk &w, uint32_t &id, double &c) {
+  auto load_ids = [&](const Walk<kK> &w, uint32_t &id, double &c) {
     const uint32_t o = w.o + (uint32_t)(bw * OW + own_l);
     id = kNone;
     c = 0.0;
@@ -334,7 +273,7 @@ __global__ void __launch_bounds__(kMul + 32 * BW, CTAS) s3ttmc_split_kernel(cons
     ep[i] = (int)(t & 0xffu) * kG3<T>;
     ez[i] = (int)(t >> 8) * kG3<T>;
   }
-  Walk w, w1;
+  Walk<kK> w, w1;
   w.start(p);
   w.open(p, zero_row);
   if (!w.valid(p)) return;
@@ -354,7 +293,7 @@ __global__ void __launch_bounds__(kMul + 32 * BW, CTAS) s3ttmc_split_kernel(cons
 #pragma unroll
     for (int q = 0; q < kVal; ++q)
       if (vdst[q] >= 0) sU[vdst[q]] = f[q] * v[q];
-    Walk w2 = w1;
+    Walk<kK> w2 = w1;
     if (w1.valid(p)) {
       load_vals(id, c, v, f);
       w2.next(p, zero_row);
@@ -501,7 +440,7 @@ void split_launch(const SplitPlan &pl, const TensorState &t, const ItemSet &item
   p.pairs = pl.pairs.p;
   p.elems = pl.elems.p;
   p.sym = pl.sym.p;
-  p.nown = t.nown;
+  p.nentries = t.nown;
   p.nrows = t.dim;
   p.nslots = t.nslots;
   if (precision == SYMPROP_FP64) dispatch<double>(p, st);

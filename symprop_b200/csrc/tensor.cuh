@@ -72,6 +72,7 @@ struct ItemSet {
   uint32_t nsplit = 0;
   uint32_t row0 = 0, rows = 0;
   bool chain = false;      // items of the pivot-chain schedule (ChainData)
+  bool groups = false;     // of its order-5 group kernel (ChainGroups)
   uint32_t nslots = 0;     // partial-sum slots of the item list
   const Chunk *light = nullptr;  // chain schedule: light rows, one chunk each
   uint32_t nlight = 0;
