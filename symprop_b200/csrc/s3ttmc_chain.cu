@@ -41,6 +41,7 @@
 #include "check.cuh"
 #include "s3ttmc_chain.cuh"
 #include "s3ttmc_chain8.cuh"
+#include "s3ttmc_mma.cuh"
 
 namespace spb {
 namespace {
@@ -455,11 +456,23 @@ __global__ void __launch_bounds__(kThreads, 4) s3ttmc_chain_kernel(const ChainPa
 // (T2[q0 q1 q2] = F[q0][q1 q2] + F[q1][q0 q2] + F[q2][q0 q1]), not one Sym3
 // per prefix.  Each thread keeps 4 x 13 entries of G (rows 4a..4a+3,
 // columns b + 64 k).
+// MMA (FP64, full batches: the rule at the launch): F and G as m8n8k4 products.  F
+// and T2 were two thirds of the CTA's time (1,080 clocks a group at R = 16: T2 went
+// through shared memory, one barrier a group).  Now four groups share a barrier, T2
+// is not stored, and its place takes batches of 64 prefixes and 16 groups.  20M
+// power-law tuples, 200,000 nodes, R = 16: 168 -> 145 ms; bound by the latency of
+// the gathers and fragment loads (8 warps an SM), the products are a third of it.
 constexpr int kThreads5 = 256;
-constexpr int kB5 = 128, kH5 = 48, kG5 = 12;
+constexpr int kB5 = 128;
+constexpr int kShort = 4;  // prefixes of a group
+template <bool MMA> constexpr int kH5 = MMA ? 64 : 48;
+template <bool MMA> constexpr int kG5 = MMA ? 16 : 12;
 constexpr int kM3 = 816;                // packed order-3 entries at R = 16
 constexpr int kS3 = kM3 + 1;            // shared row stride of G (odd: conflict-free column reads)
 constexpr int kBeta5 = (kM3 + 63) / 64;  // 13
+// F: buffers and their stride (MMA: 4 groups' fragments in different banks)
+template <bool MMA> constexpr int kFBuf = MMA ? 8 : 2;
+template <bool MMA> constexpr int kFStride = kRP * kS2 + (MMA ? 4 : 0);
 
 struct Chain5Params {
   const Chunk *chunks;
@@ -477,31 +490,36 @@ struct Chain5Params {
   uint32_t nrows, nslots;
 };
 
-template <typename T> struct Smem5 {
+template <typename T, bool MMA> struct Smem5 {
   uint32_t s1[kB5], s2[kB5], s3[kB5], s4[kB5];
   T c[kB5];
-  uint16_t h_start[kH5 + 1], g_h[kG5 + 1];
+  uint16_t h_start[kH5<MMA> + 1], g_h[kG5<MMA> + 1];
   uint32_t warp_tot[kThreads5 / 32];
   int nb, nh, ng;
   uint8_t px[kM2], py[kM2];
-  uint2 tri[kM3];
+  uint2 tri[MMA ? 1 : kM3];  // MMA: in registers
   union __align__(16) {
     struct {
-      T U3[kB5][kRP], U4[kB5][kRP];  // the owners' s_3 and s_4 rows
-      T T3[kH5][kM2];
-      T U2[kH5][kRP];
-      T T2[kG5][kM3];
-      T U1[kG5][kRP];
-      T F[2][kRP * kS2];             // F of a group (two buffers, row stride kS2)
+      union {
+        struct {
+          T U3[kB5][kRP], U4[kB5][kRP];  // the owners' s_3 and s_4 rows (until T3 is formed)
+        };
+        T F[kFBuf<MMA>][kFStride<MMA>];      // F of a group (row stride kS2)
+      };
+      T T3[kH5<MMA>][kM2];
+      T U2[kH5<MMA>][kRP];
+      T T2[MMA ? 1 : kG5<MMA>][MMA ? 2 : kM3];
+      T U1[kG5<MMA>][kRP];
     } b;
     T G[kRP * kS3];                  // the row's G at the end (row stride kS3)
   } u;
 };
 
-template <typename T>
+// MMA (FP64): F and G as products on the tensor cores
+template <typename T, bool MMA>
 __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_chain5_kernel(const Chain5Params p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  Smem5<T> &sm = *reinterpret_cast<Smem5<T> *>(smem_raw);
+  Smem5<T, MMA> &sm = *reinterpret_cast<Smem5<T, MMA> *>(smem_raw);
   const int tid = threadIdx.x;
   const Chunk ch = p.chunks[blockIdx.x];
   if (!SPB_BOUND(ch.ob <= ch.oe && ch.oe <= p.nown && ch.row < p.nrows && (ch.slot == kDirect || ch.slot < p.nslots),
@@ -520,15 +538,30 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
     sm.px[b] = (uint8_t)x;
     sm.py[b] = (uint8_t)(x + rem);
   }
-  for (uint32_t e = tid; e < m3; e += kThreads5) sm.tri[e] = p.tri[e];
+  if constexpr (!MMA)
+    for (uint32_t e = tid; e < m3; e += kThreads5) sm.tri[e] = p.tri[e];
 
-  // this thread's entries of G: rows a4 .. a4 + 3, columns bg + 64 k
+  // this thread's entries of G: rows a4 .. a4 + 3, columns bg + 64 k; MMA:
+  // 8 x 8 tiles of the tensor cores, gsum[2 i + e][k] at row 8 i + r8 and column
+  // 8 (warp + 8 k) + 2 kq + e
   const int a4 = 4 * (tid & 3), bg = tid >> 2;
+  const int warp = tid >> 5, kq = tid & 3, r8 = (tid & 31) >> 2;
+  constexpr int kWarps5 = kThreads5 / 32;
   T gsum[4][kBeta5];
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int k = 0; k < kBeta5; ++k) gsum[a][k] = T(0);
+
+  // MMA: places in F of the three terms of T2 at this lane's columns of G
+  uint2 term[MMA ? kBeta5 : 1];
+  if constexpr (MMA) {
+#pragma unroll
+    for (int k = 0; k < kBeta5; ++k) {
+      const uint32_t b = 8u * (uint32_t)(warp + kWarps5 * k) + (uint32_t)r8;
+      term[k] = b < m3 ? p.tri[b] : make_uint2(0u, 0u);
+    }
+  }
 
   // owner record of window slot tid (tid < kB5), prefetched a batch ahead
   uint4 rid = make_uint4(0, 0, 0, 0);
@@ -561,7 +594,7 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
       fl = (f & 1u) | (((f >> 1) & 1u) << 16);
     }
     const uint32_t cnt = cta_scan(fl, sm.warp_tot);  // inclusive: groups | prefixes << 16
-    auto within = [](uint32_t c) { return (c & 0xffffu) <= (uint32_t)kG5 && (c >> 16) <= (uint32_t)kH5; };
+    auto within = [](uint32_t c) { return (c & 0xffffu) <= (uint32_t)kG5<MMA> && (c >> 16) <= (uint32_t)kH5<MMA>; };
     const bool v = in && within(cnt);
     const bool prev_valid = tid > 0 && tid <= kB5 && (uint64_t)(tid - 1) < left && within(cnt - fl);
     if (!v && prev_valid) sm.nb = tid;
@@ -642,7 +675,98 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
     //         r4 .. r4 + 3 and columns c + 64 j of it per thread)
     //   T2_g[q0 q1 q2] = F_g[q0][q1 q2] + F_g[q1][q0 q2] + F_g[q2][q0 q1]
     // F alternates between two buffers, so one barrier per group suffices.
-    {
+    // MMA: four groups at a time, two warps each, F as 8 x 8 x 4 products over
+    // the prefixes.  T2 is not stored: the lane that multiplies an entry of it
+    // adds its three terms from F.  The products of G with four groups and the F
+    // of the next four share a barrier interval (eight buffers).
+    if constexpr (MMA) {
+      auto form_f = [&](int g0) {
+        int longest = 0;
+        for (int g = g0; g < min(g0 + 4, ng); ++g) longest = max(longest, sm.g_h[g + 1] - sm.g_h[g]);
+        if (g0 + 4 <= ng && longest <= kShort) {
+          // four groups of few prefixes: two warps each, column tiles warp % 2 + 2 k
+          const int g = g0 + (warp >> 1);
+          constexpr int kN = (kM2 / 8 + 1) / 2;
+          double f[kN][2][2];
+#pragma unroll
+          for (int k = 0; k < kN; ++k) f[k][0][0] = f[k][0][1] = f[k][1][0] = f[k][1][1] = 0.0;
+          const int h1 = sm.g_h[g + 1];
+          for (int h = sm.g_h[g] + kq; h - kq < h1; h += 4) {
+            const bool on = h < h1;
+            double u[2], t[kN];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) u[i] = on ? sm.u.b.U2[h][8 * i + r8] : 0.0;
+#pragma unroll
+            for (int k = 0; k < kN; ++k) {
+              const int j = (warp & 1) + 2 * k;
+              t[k] = on && j < kM2 / 8 ? sm.u.b.T3[h][8 * j + r8] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kN; ++k)
+#pragma unroll
+              for (int i = 0; i < 2; ++i) mma_f64(f[k][i], u[i], t[k]);
+          }
+          T *F = sm.u.b.F[g & 7];
+#pragma unroll
+          for (int k = 0; k < kN; ++k) {
+            const int j = (warp & 1) + 2 * k;
+            if (8 * j >= (int)m2) break;
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+              for (int e = 0; e < 2; ++e) F[(8 * i + r8) * kS2 + 8 * j + 2 * kq + e] = f[k][i][e];
+          }
+          return;
+        }
+        // else one group after the other, all warps: tiles warp + 8 k of the 2 x 17
+        constexpr int kN = (2 * kM2 / 8 + kWarps5 - 1) / kWarps5;
+        for (int g = g0; g < min(g0 + 4, ng); ++g) {
+          double f[kN][2];
+#pragma unroll
+          for (int k = 0; k < kN; ++k) f[k][0] = f[k][1] = 0.0;
+          const int h1 = sm.g_h[g + 1];
+          for (int h = sm.g_h[g] + kq; h - kq < h1; h += 4) {
+            const bool on = h < h1;
+            const double a = on ? sm.u.b.U2[h][8 * (warp & 1) + r8] : 0.0;
+            double t[kN];
+#pragma unroll
+            for (int k = 0; k < kN; ++k) {
+              const int j = (warp + kWarps5 * k) >> 1;
+              t[k] = on && j < kM2 / 8 ? sm.u.b.T3[h][8 * j + r8] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kN; ++k)
+              if (warp + kWarps5 * k < 2 * kM2 / 8) mma_f64(f[k], a, t[k]);
+          }
+          T *F = sm.u.b.F[g & 7];
+#pragma unroll
+          for (int k = 0; k < kN; ++k) {
+            const int j = (warp + kWarps5 * k) >> 1;
+            if (8 * j >= (int)m2) break;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) F[(8 * (warp & 1) + r8) * kS2 + 8 * j + 2 * kq + e] = f[k][e];
+          }
+        }
+      };
+      form_f(0);
+      for (int g0 = 0; g0 < ng; g0 += 4) {
+        __syncthreads();
+        const int g = g0 + kq;
+        const bool on = g < ng;
+        const T *F = sm.u.b.F[g & 7];
+        double u[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) u[i] = on ? sm.u.b.U1[g][8 * i + r8] : 0.0;
+#pragma unroll
+        for (int k = 0; k < kBeta5; ++k) {
+          if (8 * (warp + kWarps5 * k) >= (int)m3) break;
+          const double t2 = on ? F[term[k].x & 0xffffu] + F[term[k].x >> 16] + F[term[k].y] : 0.0;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) mma_f64(gsum[2 * i][k], gsum[2 * i + 1][k], u[i], t2);
+        }
+        form_f(g0 + 4);
+      }
+    } else {
       const int r4 = 4 * (tid & 3), c0 = tid >> 2;
       for (int g = 0; g < ng; ++g) {
         T f[4][3];
@@ -680,16 +804,18 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
     }
     __syncthreads();
     // ---- G += U1_g (x) T2_g over the batch's groups
-    for (int g = 0; g < ng; ++g) {
-      T u[4];
+    if constexpr (!MMA) {
+      for (int g = 0; g < ng; ++g) {
+        T u[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) u[a] = sm.u.b.U1[g][a4 + a];
+        for (int a = 0; a < 4; ++a) u[a] = sm.u.b.U1[g][a4 + a];
 #pragma unroll
-      for (int k = 0; k < kBeta5; ++k) {
-        const int b = bg + 64 * k;
-        const T t2 = b < (int)m3 ? sm.u.b.T2[g][b] : T(0);
+        for (int k = 0; k < kBeta5; ++k) {
+          const int b = bg + 64 * k;
+          const T t2 = b < (int)m3 ? sm.u.b.T2[g][b] : T(0);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) gsum[a][k] += u[a] * t2;
+          for (int a = 0; a < 4; ++a) gsum[a][k] += u[a] * t2;
+        }
       }
     }
     o0 += (uint64_t)nb;
@@ -701,8 +827,9 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int k = 0; k < kBeta5; ++k) {
-      const int b = bg + 64 * k;
-      if (b < kM3) sG[(a4 + a) * kS3 + b] = gsum[a][k];
+      const int x = MMA ? 8 * (a >> 1) + r8 : a4 + a,
+                b = MMA ? 8 * (warp + kWarps5 * k) + 2 * kq + (a & 1) : bg + 64 * k;
+      if (b < kM3) sG[x * kS3 + b] = gsum[a][k];
     }
   __syncthreads();
   T *Yrow = reinterpret_cast<T *>(p.Y) + (uint64_t)ch.row * p.m4;
@@ -1122,17 +1249,17 @@ void chain5_rows_launch(const TensorState &t, const ChainData &cd, const ItemSet
   p.nown = t.nown;
   p.nrows = t.dim;
   p.nslots = items.nslots;
-  if (precision == SYMPROP_FP64) {
-    const size_t smem = sizeof(Smem5<double>);
-    SPB_CUDA(cudaFuncSetAttribute(s3ttmc_chain5_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    s3ttmc_chain5_kernel<double><<<items.nchunks, kThreads5, smem, st>>>(p);
-  } else {
-    const size_t smem = sizeof(Smem5<float>);
-    SPB_CUDA(cudaFuncSetAttribute(s3ttmc_chain5_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    s3ttmc_chain5_kernel<float><<<items.nchunks, kThreads5, smem, st>>>(p);
-  }
+  auto go = [&](auto kern, size_t smem) {
+    SPB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<items.nchunks, kThreads5, smem, st>>>(p);
+  };
+  // The products pay where batches are full: 64 owners a node on average.  R = 16, ms,
+  // without / with: 500 owners a node (2M tuples) 13.25 / 11.75, 200 (200,000)
+  // 1.335 / 1.274, 25 (100,000) 1.70 / 1.69, 10 (200,000) 5.92 / 6.00, 2.5 (100,000)
+  // 9.49 / 9.73.
+  if (precision != SYMPROP_FP64) go(s3ttmc_chain5_kernel<float, false>, sizeof(Smem5<float, false>));
+  else if (t.nown >= 64ull * t.dim) go(s3ttmc_chain5_kernel<double, true>, sizeof(Smem5<double, true>));
+  else go(s3ttmc_chain5_kernel<double, false>, sizeof(Smem5<double, false>));
   SPB_LAUNCH_CHECK();
   spb_check_host(st, "S3TTMc chain kernel (order 5)");
 }

@@ -19,11 +19,12 @@ template <int THREADS> __device__ __forceinline__ void bar_arrive(int id) {
 
 // c (8 x 8, rows r8 = lane / 4, columns 2 kq + {0, 1}, kq = lane % 4) +=
 // a (8 x 4: row r8, column kq) * b (4 x 8: row kq, column r8)
-__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) {
+__device__ __forceinline__ void mma_f64(double &c0, double &c1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(c[0]), "+d"(c[1])
+               : "+d"(c0), "+d"(c1)
                : "d"(a), "d"(b));
 }
+__device__ __forceinline__ void mma_f64(double (&c)[2], double a, double b) { mma_f64(c[0], c[1], a, b); }
 
 // (d0, d1) += (a, a) * (b0, b1) in one paired FP32 FMA: each half rounds as a
 // scalar fmaf does
