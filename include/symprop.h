@@ -168,7 +168,8 @@ int symprop_unpack_rows_device(const double *dpacked, uint64_t rows,
  * src/dense/matrixops.cpp:18-43; symsyrk :126-146 is its n x n twin).
  * precision SYMPROP_FP64: dY, dscale are double*; from 1,536 rows and 320
  * columns on integer tensor cores (exact sums of the columns rounded to 53
- * bits of their largest entry), else FP64 CUDA-core GEMM;
+ * bits of their largest entry) where that keeps every entry within the rounding
+ * bound of an FP64 sum, n 2^-53 sum_k |y_ki| |y_kj|, else FP64 CUDA-core GEMM;
  * SYMPROP_FP32: dY, dscale are float*, tcgen05 tensor cores with split-BF16
  * operands and FP32 accumulation. */
 int symprop_gram_device(const void *dY, uint64_t n, uint32_t m, const void *dscale,

@@ -265,8 +265,7 @@ int symprop_gram_device(const void *dY, uint64_t n, uint32_t m, const void *dsca
     cudaStream_t st = (cudaStream_t)stream;
     if (precision == SYMPROP_FP64) {
       const double *Y = (const double *)dY, *sd = (const double *)dscale;
-      dense::gemm<double>(st, (int)m, (int)m, (int)n, 1.0, Y, (int)m, true, Y, (int)m, false, 0.0, dG,
-                          (int)m, nullptr, true);
+      dense::gram_cols(st, Y, (int)n, (int)m, dG, dense::GramUse::kEntries);
       dense::scale_sym(st, dG, (int)m, sd);
     } else if (precision == SYMPROP_FP32) {
       PoolBuf ws(gram::workspace_bytes((int)n, (int)m), st);

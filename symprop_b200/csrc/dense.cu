@@ -908,13 +908,10 @@ void gemm(cudaStream_t st, int M, int N, int K, T alpha, const T *A, int lda, bo
       SPB_LAUNCH_CHECK();
       return;
     }
-    if (transA && !transB && sym_upper && A == B && lda == ldb && M == N && !kscale && alpha == 1.0 && beta == 0.0) {
-      // a column Gram: the integer tensor cores where they pay and A is finite
-      if (gram::i8_gram_pays(K, M) && gram::gram_cols_i8(st, A, K, M, lda, C, ldc)) return;
-      if (M >= GB && M % 2 == 0 && lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0) {
-        gram_f64(st, M, K, A, lda, C, ldc);
-        return;
-      }
+    if (transA && !transB && sym_upper && A == B && lda == ldb && M == N && !kscale && M >= GB && M % 2 == 0 &&
+        lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && alpha == 1.0 && beta == 0.0) {
+      gram_f64(st, M, K, A, lda, C, ldc);
+      return;
     }
   }
   const int nb = N <= 32 && !sym_upper ? 32 : 64;
@@ -1010,6 +1007,12 @@ void householder_q(cudaStream_t st, double *A, int rows, int cols) {
   householder_kernel<<<1, 1024, 0, st>>>(A, rows, cols, tau.as<double>(), Q.as<double>());
   SPB_LAUNCH_CHECK();
   SPB_CUDA(cudaMemcpyAsync(A, Q.p, sizeof(double) * (size_t)rows * cols, cudaMemcpyDeviceToDevice, st));
+}
+
+void gram_cols(cudaStream_t st, const double *A, int rows, int cols, double *C, GramUse use) {
+  if (gram::i8_gram_pays(rows, cols) && gram::gram_cols_i8(st, A, rows, cols, cols, C, cols, use == GramUse::kEntries))
+    return;
+  gemm<double>(st, cols, cols, rows, 1.0, A, cols, true, A, cols, false, 0.0, C, cols, nullptr, true);
 }
 
 // CholQR2 calls that fell back to Householder QR (reported by the trace)

@@ -21,6 +21,13 @@ void gemm(cudaStream_t st, int M, int N, int K, T alpha, const T *A, int lda, bo
           const T *B, int ldb, bool transB, T beta, T *C, int ldc, const T *kscale = nullptr,
           bool sym_upper = false);
 
+// C (cols x cols, full symmetric) = A^T A for a row-major rows x cols FP64 A, on the
+// integer tensor cores where they pay (gram_i8.cuh), else gemm.  kEntries: every
+// entry within the rounding bound of an FP64 sum.  kSpectrum, for eigenvalue
+// problems: every entry within that of |a_i| |a_j|.
+enum class GramUse { kEntries, kSpectrum };
+void gram_cols(cudaStream_t st, const double *A, int rows, int cols, double *C, GramUse use);
+
 // core (r x m, FP64) = U^T Y for FP64 U (n x r) and FP32 Y (n x m), both
 // row-major: Y is read once and widened in registers, FP64 accumulation,
 // deterministic (fixed row chunks summed in order).

@@ -17,6 +17,23 @@
 // 2^-54 of the column maximum per entry with random sign, and of one rounding
 // per chunk.
 //
+// What the rounding may cost an entry.  With P_j = 2^(53 - s_j) (the power of
+// two above column j's largest magnitude of a chunk) the entry (i, j) is off by at
+// most 2^-54 sum_k (|a_ki| P_j + |a_kj| P_i): small against |a_i| |a_j|, which is
+// all that an eigenvalue problem asks for, but not against
+// T_ij = sum_k |a_ki| |a_kj|, the scale of a sum in floating point, where the
+// columns' large entries lie in different rows.  A caller that wants every
+// entry (componentwise) gets this checked first: |a_kj| / P_j in 7 bits, rounded
+// down, gives a lower bound W of T / (P_i P_j) by one more product, and with
+// N_j = |a_j| / P_j (2-norm) an entry is kept where
+//     N_i + N_j <= sqrt(rows of the chunk) W      in every chunk.
+// Then sum |a_ki| <= sqrt(rows) N_i P_i makes its error at most
+// rows / 2 * 2^-53 T_ij, half the bound of a sum of `rows` terms in floating
+// point, and (the roundings having random signs) 0.3 sqrt(rows) 2^-53 T_ij in the
+// root mean square, what a floating-point sum of terms of one sign is off by.
+// The other entries are summed in FP64 (pair_kernel), or all of them by the
+// caller when they are many.
+//
 // Bound: 16 int8 products over the upper 256 x 256 tiles.  200,000 x 3,876:
 // 136 tiles, 5.7e13 integer operations (12.7 ms at the nominal 4.5 POP/s),
 // against 3.0e12 FP64 operations (81 ms at the nominal 37 TFLOP/s) for the
@@ -105,49 +122,101 @@ __global__ void scale_kernel(const unsigned long long *cmax, int n, int *s, int 
   s[i] = b ? 53 - e : 0;
 }
 
-// Residues of the scaled columns: out[(chunk * 16 + p) * cols + c][k], k < kc
+// Residues of the scaled columns: out[(chunk * planes + p) * cols + c][k], k < kc
 // bytes contiguous (rows past the chunk's end are zero).  A thread takes 32
 // rows of one column: a warp reads 256-byte row pieces, and every store fills a
-// 32-byte sector.  q = round(n / p) is within 2^-7 of n / p + 1/2, so |r| may
-// pass p / 2 by 2: put back into 8 bits where p / 2 + 2 > 127.
+// 32-byte sector.  q = round(n / p) is within 2^-7 of n / p + 1/2, so |r|
+// may pass p / 2 by 2: put back into 8 bits where p / 2 + 2 > 127.
+// MAG: the last plane takes |n| 2^-53 in 7 bits, rounded down, and nsq the sum of
+// the squares of the same in 15 bits, rounded up (integers: the decision that
+// rests on them is the same in every run).
+template <bool MAG>
 __global__ void __launch_bounds__(128) residue_kernel(const double *__restrict__ A, int rows, int cols, int lda,
                                                       int chunk, int kc, const int *__restrict__ s, int chunk0,
-                                                      signed char *__restrict__ out) {
-  const int c = blockIdx.x * 32 + (threadIdx.x & 31);
-  const int k0 = blockIdx.y * 128 + (threadIdx.x >> 5) * 32;  // within the chunk
-  if (c >= cols) return;
+                                                      signed char *__restrict__ out,
+                                                      unsigned long long *__restrict__ nsq) {
+  constexpr int kPlanes = kP + (MAG ? 1 : 0);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+  const int k0 = blockIdx.y * 128 + warp * 32;  // within the chunk
   const int ch = chunk0 + blockIdx.z;
-  const int r0 = ch * chunk + k0, r1 = min(rows, (ch + 1) * chunk);
-  const int sh = s[(size_t)ch * cols + c], s1 = sh / 2;
-  // 2^sh as two factors: sh may lie outside the exponent range
-  const double f1 = __longlong_as_double((long long)(s1 + 1023) << 52),
-               f2 = __longlong_as_double((long long)(sh - s1 + 1023) << 52);
-  constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
-  double n[32];
+  unsigned long long sum = 0;
+  if (c < cols) {
+    const int r0 = ch * chunk + k0, r1 = min(rows, (ch + 1) * chunk);
+    const int sh = s[(size_t)ch * cols + c], s1 = sh / 2;
+    // 2^sh as two factors: sh may lie outside the exponent range
+    const double f1 = __longlong_as_double((long long)(s1 + 1023) << 52),
+                 f2 = __longlong_as_double((long long)(sh - s1 + 1023) << 52);
+    constexpr double kMagic = 6755399441055744.0;  // 1.5 * 2^52: adding it rounds to an integer
+    double n[32];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) n[i] = r0 + i < r1 ? rint(A[(size_t)(r0 + i) * lda + c] * f1 * f2) : 0.0;
-  for (int p = 0; p < kP; ++p) {
-    const double m = (double)c_mod[p], rm = c_crt.rp[p];
-    uint32_t w[8];
+    for (int i = 0; i < 32; ++i) n[i] = r0 + i < r1 ? rint(A[(size_t)(r0 + i) * lda + c] * f1 * f2) : 0.0;
+    signed char *plane = out + ((size_t)blockIdx.z * kPlanes * cols + c) * kc + k0;
+    auto store = [&](int p, const uint32_t (&w)[8]) {
+      uint4 *o = reinterpret_cast<uint4 *>(plane + (size_t)p * cols * kc);
+      o[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    };
+    for (int p = 0; p < kP; ++p) {
+      const double m = (double)c_mod[p], rm = c_crt.rp[p];
+      uint32_t w[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      uint32_t v = 0;
+      for (int q = 0; q < 8; ++q) {
+        uint32_t v = 0;
 #pragma unroll
-      for (int b = 0; b < 4; ++b) {
-        const double x = n[4 * q + b];
-        const double t = fma(x, rm, kMagic) - kMagic;
-        int r = (int)__double_as_longlong(fma(-t, m, x) + kMagic);  // the low word holds the integer
-        if (p == 1 || p == 2) {  // 255, 253 (for 256 the byte wraps to the same residue)
-          const int mi = c_mod[p];
-          r = r > 127 ? r - mi : r < -128 ? r + mi : r;
+        for (int b = 0; b < 4; ++b) {
+          const double x = n[4 * q + b];
+          const double t = fma(x, rm, kMagic) - kMagic;
+          int r = (int)__double_as_longlong(fma(-t, m, x) + kMagic);  // the low word holds the integer
+          if (p == 1 || p == 2) {  // 255, 253 (for 256 the byte wraps to the same residue)
+            const int mi = c_mod[p];
+            r = r > 127 ? r - mi : r < -128 ? r + mi : r;
+          }
+          v |= (uint32_t)(r & 0xff) << (8 * b);
         }
-        v |= (uint32_t)(r & 0xff) << (8 * b);
+        w[q] = v;
       }
-      w[q] = v;
+      store(p, w);
     }
-    uint4 *o = reinterpret_cast<uint4 *>(out + ((size_t)(blockIdx.z * kP + p) * cols + c) * kc + k0);
-    o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-    o[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    if constexpr (MAG) {
+      uint32_t w[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        w[q] = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const float x = fabsf((float)n[4 * q + b]) * 0x1p-53f;
+          w[q] |= (uint32_t)min((int)(x * 127.f), 127) << (8 * b);
+          const uint32_t u = (uint32_t)ceilf(x * 32768.f);
+          sum += (unsigned long long)u * u;
+        }
+      }
+      store(kP, w);
+    }
+  }
+  if constexpr (MAG) {
+    __shared__ unsigned long long part[4][32];
+    part[warp][lane] = sum;
+    __syncthreads();
+    if (warp == 0 && c < cols)
+      atomicAdd(&nsq[(size_t)ch * cols + c], part[0][lane] + part[1][lane] + part[2][lane] + part[3][lane]);
+  }
+}
+
+// The entries (i, j) of the list in FP64: C_ij = C_ji = sum_k a_ki a_kj
+__global__ void __launch_bounds__(256) pair_kernel(const int2 *__restrict__ pairs, const double *__restrict__ A,
+                                                   int rows, int lda, double *__restrict__ C, int ldc) {
+  __shared__ double red[8];
+  const int2 p = pairs[blockIdx.x];
+  double sum = 0.0;
+#pragma unroll 4
+  for (int k = threadIdx.x; k < rows; k += 256) sum = fma(A[(size_t)k * lda + p.x], A[(size_t)k * lda + p.y], sum);
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) sum += red[w];
+    C[(size_t)p.x * ldc + p.y] = sum;
+    C[(size_t)p.y * ldc + p.x] = sum;
   }
 }
 
@@ -167,10 +236,16 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 struct I8Args {
   int cols, ntile, ntiles;    // tiles of 256 per side, upper tiles
   int kblocks;                // 128-wide blocks of a chunk
-  unsigned char *C;           // (chunk * 16 + p) planes of ld x ld residues
+  unsigned char *C;           // (chunk * kP + p) planes of ld x ld residues
   int ld;
   int *err;
   uint64_t wait_ns;
+  int planes;                 // per chunk: kP of residues, one more of magnitudes
+  // magnitudes: entries to be summed in FP64 go to the list
+  const unsigned long long *nsq;
+  int chunk0, chunk, rows;
+  int2 *pairs;
+  unsigned *npairs, max_pairs;
 };
 
 __global__ void __launch_bounds__(256, 1)
@@ -203,6 +278,14 @@ __global__ void __launch_bounds__(256, 1)
     abort_flag = 0;
     progress = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  const int chunk = a.chunk0 + plane / a.planes, modulus = plane % a.planes;
+  const bool check = modulus == kP;
+  __shared__ float norm[kTile];  // check: N of the tile's columns, 0 past the last
+  const unsigned long long *nsq = a.nsq + (size_t)chunk * a.cols;
+  if (check) {
+    const int j = tj * kTile + threadIdx.x;
+    norm[threadIdx.x] = j < a.cols ? sqrtf((float)nsq[j]) * 0x1p-15f : 0.f;
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
@@ -256,13 +339,34 @@ __global__ void __launch_bounds__(256, 1)
   const bool done = mbar_wait_progress(&done_bar, &progress);
   asm volatile("tcgen05.fence::after_thread_sync;");
   const int go = __all_sync(0xffffffffu, done ? 1 : 0) && !__shfl_sync(0xffffffffu, (int)abort_flag, 0);
-  if (go) {
+  if (go && check) {
+    const int half = warp >> 2, i = ti * kTile + half * 128 + (warp & 3) * 32 + lane;
+    const float ni = i < a.cols ? sqrtf((float)nsq[i]) * 0x1p-15f : 0.f;
+    const float unit = sqrtf((float)min(a.chunk, a.rows - chunk * a.chunk)) / (127.f * 127.f);
+#pragma unroll 1
+    for (int c = 0; c < kTile; c += 32) {
+      uint32_t v[32];
+      tmem_load<32>(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(half * 256 + c), v);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int q = 0; q < 32; ++q) {
+        const float nj = norm[c + q];
+        const int j = tj * kTile + c + q;
+        if (ni > 0.f && nj > 0.f && i <= j && !(ni + nj <= unit * (float)(int)v[q])) {
+          // past the limit the count no longer matters (and may not wrap)
+          if (*(volatile unsigned *)a.npairs > a.max_pairs) continue;
+          const unsigned at = atomicAdd(a.npairs, 1u);
+          if (at < a.max_pairs) a.pairs[at] = make_int2(i, j);
+        }
+      }
+    }
+  } else if (go) {
     // warp w: lanes of quadrant w % 4 of accumulator w / 4.  The sums (at most
     // 2^30 in magnitude) modulo p, times (P / p)^-1 modulo p.
     const int half = warp >> 2, r = ti * kTile + half * 128 + (warp & 3) * 32 + lane;
-    const uint32_t p = (uint32_t)c_mod[plane % kP], inv = c_crt.inv[plane % kP];
+    const uint32_t p = (uint32_t)c_mod[modulus], inv = c_crt.inv[modulus];
     const uint32_t magic = 0xffffffffu / p, bias = (1u << 30) / p * p + p;
-    unsigned char *C = a.C + (size_t)plane * a.ld * a.ld + (size_t)r * a.ld + tj * kTile;
+    unsigned char *C = a.C + (size_t)(plane / a.planes * kP + modulus) * a.ld * a.ld + (size_t)r * a.ld + tj * kTile;
 #pragma unroll 1
     for (int c = 0; c < kTile; c += 32) {
       uint32_t v[32];
@@ -413,6 +517,7 @@ I8Plan plan_i8(int rows, int cols) {
     }
   }
   g.group = std::min(g.group, g.nchunk);
+  g.chunk = (rows + g.nchunk - 1) / g.nchunk;  // chunks of like length: no short last one
   return g;
 }
 
@@ -442,13 +547,22 @@ struct Pool {  // scratch from the library's stream-ordered pool
 // either way).
 bool i8_gram_pays(int rows, int cols) { return cols >= 320 && rows >= 1536; }
 
-bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc) {
+// Entries that the caller of a componentwise Gram may have summed one by one: 64
+// bytes of A a row each, against cols^2 / 2 FMAs a row for all of them by the FP64
+// kernel (equal at about cols^2 / 900); a few odd columns always.
+static unsigned max_pairs(int cols) {
+  return (unsigned)std::max<long long>(4ll * cols, (long long)cols * cols / 1024);
+}
+
+bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc,
+                  bool componentwise) {
   const I8Plan g = plan_i8(rows, cols);
   const size_t ncs = (size_t)g.nchunk * cols;
-  Pool cmax(ncs * 8, st), sc(ncs * 4, st), flags(2 * sizeof(int), st);
+  Pool cmax(ncs * 8, st), sc(ncs * 4, st), flags(3 * sizeof(int), st);
   int *bad = (int *)flags.p, *err = bad + 1;
+  unsigned *npairs = (unsigned *)(bad + 2);
   SPB_CUDA(cudaMemsetAsync(cmax.p, 0, ncs * 8, st));
-  SPB_CUDA(cudaMemsetAsync(flags.p, 0, 2 * sizeof(int), st));
+  SPB_CUDA(cudaMemsetAsync(flags.p, 0, 3 * sizeof(int), st));
   const int part = 512;
   col_max_kernel<<<dim3((cols + 127) / 128, g.nchunk, (g.chunk + part - 1) / part), 128, 0, st>>>(
       A, rows, cols, lda, g.chunk, part, (unsigned long long *)cmax.p);
@@ -456,29 +570,42 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
   scale_kernel<<<(unsigned)((ncs + 255) / 256), 256, 0, st>>>((const unsigned long long *)cmax.p, (int)ncs,
                                                               (int *)sc.p, bad);
   SPB_LAUNCH_CHECK();
-  int h[2] = {0, 0};
-  SPB_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
-  SPB_CUDA(cudaStreamSynchronize(st));
-  if (h[0]) return false;
-  SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+  int h[3] = {0, 0, 0};
+  auto read_flags = [&] {  // false: A is left to the FP64 kernel
+    SPB_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
+    SPB_CUDA(cudaStreamSynchronize(st));
+    if (h[1]) fail(SYMPROP_ERR_TIMEOUT, "integer tensor-core Gram: a bounded wait expired");
+    return !h[0] && (unsigned)h[2] <= max_pairs(cols);
+  };
+  if (!read_flags()) return false;
+  // The check of a componentwise Gram runs with the residues and their product.  Before
+  // them it would cost less where the FP64 kernel has the last word (200,000 x 3,876:
+  // 4 instead of 28 of 165 ms) and more everywhere else (29.8 instead of 28.2 ms;
+  // 10,000 x 816: 0.443 instead of 0.409 ms; without a check 27.2 and 0.405 ms).
+  const int planes = kP + (componentwise ? 1 : 0);
   Pool res(st), rem(st);
-  if (!res.take_operands((size_t)g.group * kP * cols * g.kc) || !rem.take_operands((size_t)g.group * kP * g.ld * g.ld))
+  if (!res.take_operands((size_t)g.group * planes * cols * g.kc) ||
+      !rem.take_operands((size_t)g.group * kP * g.ld * g.ld))
     return false;
+  Pool list(componentwise ? max_pairs(cols) * sizeof(int2) : 0, st), nsq(componentwise ? ncs * 8 : 0, st);
+  if (componentwise) SPB_CUDA(cudaMemsetAsync(nsq.p, 0, ncs * 8, st));
+  SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   for (int c0 = 0; c0 < g.nchunk; c0 += g.group) {
     const int nc = std::min(g.group, g.nchunk - c0);
-    residue_kernel<<<dim3((cols + 31) / 32, g.kc / 128, nc), 128, 0, st>>>(A, rows, cols, lda, g.chunk, g.kc,
-                                                                          (const int *)sc.p, c0,
-                                                                          (signed char *)res.p);
+    auto residues = componentwise ? residue_kernel<true> : residue_kernel<false>;
+    residues<<<dim3((cols + 31) / 32, g.kc / 128, nc), 128, 0, st>>>(A, rows, cols, lda, g.chunk, g.kc,
+                                                                     (const int *)sc.p, c0, (signed char *)res.p,
+                                                                     (unsigned long long *)nsq.p);
     SPB_LAUNCH_CHECK();
     CUtensorMap map;
-    cuuint64_t dims[2] = {(cuuint64_t)g.kc, (cuuint64_t)nc * kP * cols};
+    cuuint64_t dims[2] = {(cuuint64_t)g.kc, (cuuint64_t)nc * planes * cols};
     cuuint64_t strides[1] = {(cuuint64_t)g.kc};
     cuuint32_t box[2] = {kBK, kTile}, estr[2] = {1, 1};
     const CUresult r = get_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, res.p, dims, strides, box, estr,
                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) fail(SYMPROP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    I8Args a;
+    I8Args a{};
     a.cols = cols;
     a.ntile = g.ntile;
     a.ntiles = g.ntiles;
@@ -487,16 +614,26 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     a.ld = g.ld;
     a.err = err;
     a.wait_ns = mainloop_wait_ns();
-    i8_gram_kernel<<<(unsigned)(g.ntiles * kP * nc), 256, kSmem, st>>>(map, a);
+    a.planes = planes;
+    a.nsq = (const unsigned long long *)nsq.p;
+    a.chunk0 = c0;
+    a.chunk = g.chunk;
+    a.rows = rows;
+    a.pairs = (int2 *)list.p;
+    a.npairs = npairs;
+    a.max_pairs = max_pairs(cols);
+    i8_gram_kernel<<<(unsigned)(g.ntiles * planes * nc), 256, kSmem, st>>>(map, a);
     SPB_LAUNCH_CHECK();
     const unsigned nt = (unsigned)((cols + 31) / 32);
     crt_kernel<<<dim3(nt, nt), 256, 0, st>>>((const unsigned char *)rem.p, g.ld, cols, nc, c0, (const int *)sc.p,
                                              c0 > 0 ? 1 : 0, C, ldc);
     SPB_LAUNCH_CHECK();
   }
-  SPB_CUDA(cudaMemcpyAsync(h, flags.p, sizeof(h), cudaMemcpyDeviceToHost, st));
-  SPB_CUDA(cudaStreamSynchronize(st));
-  if (h[1]) fail(SYMPROP_ERR_TIMEOUT, "integer tensor-core Gram: a bounded wait expired");
+  if (!read_flags()) return false;
+  if (const unsigned odd = (unsigned)h[2]) {
+    pair_kernel<<<odd, 256, 0, st>>>((const int2 *)list.p, A, rows, lda, C, ldc);
+    SPB_LAUNCH_CHECK();
+  }
   return true;
 }
 

@@ -10,10 +10,15 @@ namespace gram {
 // tensor cores.
 bool i8_gram_pays(int rows, int cols);
 // C (cols x cols, full symmetric, row stride ldc) = A^T A for a row-major
-// rows x cols FP64 A (row stride lda).  False, with C untouched, when A holds
-// an infinity or a NaN, or when there is no device memory for the operands (at
-// most about 4.5 GB, from the library's pool).  Waits for `st`.
-bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc);
+// rows x cols FP64 A (row stride lda), each entry within about 2^-53 |a_i| |a_j|
+// (columns of A).  componentwise: within rows * 2^-53 sum_k |a_ki| |a_kj| as well,
+// the bound of a sum in FP64.  False when A holds an infinity
+// or a NaN, when a componentwise Gram has many columns whose large entries lie
+// in different rows, or when there is no device memory for the operands (at
+// most about 4.5 GB, from the library's pool).  Waits for `st`,
+// except for the last sums of odd entries.
+bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc,
+                  bool componentwise);
 
 }  // namespace gram
 }  // namespace spb

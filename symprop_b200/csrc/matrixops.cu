@@ -187,8 +187,7 @@ int symprop_leftsvd(const double *A, double *U, uint64_t nr, uint64_t nc, uint64
       // (they are orthogonal with norms sigma_j; CholQR keeps each column's
       // direction)
       DBuf<double> G(nc * nc), V(nc * rank);
-      dense::gemm<double>(0, (int)nc, (int)nc, (int)nr, 1.0, dA.p, (int)nc, true, dA.p, (int)nc, false, 0.0, G.p,
-                          (int)nc, nullptr, true);
+      dense::gram_cols(0, dA.p, (int)nr, (int)nc, G.p, dense::GramUse::kSpectrum);
       st = top_eigvecs(G.p, (int)nc, (int)rank, V.p);
       dense::gemm<double>(0, (int)nr, (int)rank, (int)nc, 1.0, dA.p, (int)nc, false, V.p, (int)rank, false, 0.0,
                           dU.p, (int)rank);

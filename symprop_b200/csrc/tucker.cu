@@ -281,7 +281,8 @@ int run_tucker(TensorState &t, const symprop_config &c, int alg, symprop_result 
           gram::split(st, Y32.p, sD32.p, Z);
           gram::gram_cols(st, Z, S.p, gram_scr.p, gram_err.p);
         } else {
-          dense::gemm<double>(st, m, m, n, 1.0, Y.p, m, true, Y.p, m, false, 0.0, S.p, m, nullptr, true);
+          // (only the leading eigenvectors of S are used)
+          dense::gram_cols(st, Y.p, n, m, S.p, dense::GramUse::kSpectrum);
           scale_sym_kernel<<<(unsigned)(((size_t)m * m + 255) / 256), 256, 0, st>>>(S.p, m, dsD.p);
           SPB_LAUNCH_CHECK();
         }
