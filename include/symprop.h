@@ -215,6 +215,11 @@ int symprop_symgemm_device(const float *dA, const double *dB, const double *dsca
  * restores the default.  A wait that expires ends the call with
  * SYMPROP_ERR_TIMEOUT after the kernel has drained what it issued. */
 int symprop_debug_set_tc_wait_ns(uint64_t ns);
+/* Further failure injection for tests, for the whole process; 0 switches a key off.
+ *   SYMPROP_DEBUG_TC_EXPIRED_WARP  w + 1: warp w of every tensor-core Gram CTA takes
+ *                                  its wait for the sums as expired */
+enum { SYMPROP_DEBUG_TC_EXPIRED_WARP = 0, SYMPROP_DEBUG_KEYS };
+int symprop_debug_set(int key, uint64_t value);
 
 /* ------------------------------------------- matrix:: operations (host) */
 /* FP64 row-major matrices in host memory, computed on the current device:

@@ -103,6 +103,7 @@ def lib():
         "symprop_symsyrk_device": (_I, [_P, _P, _P, _U64, _U64, _P]),
         "symprop_symgemm_device": (_I, [_P, _P, _P, _P, _U64, _U64, _U64, _P]),
         "symprop_debug_set_tc_wait_ns": (_I, [_U64]),
+        "symprop_debug_set": (_I, [_I, _U64]),
         "symprop_tensor_load_tns": (_I, [ctypes.c_char_p, ctypes.POINTER(_P)]),
         "symprop_tensor_copy_nonzeros": (_I, [_P, _P, _P]),
         "symprop_tensor_load_spt": (_I, [ctypes.c_char_p, ctypes.POINTER(_P)]),
@@ -136,6 +137,7 @@ def exported_symbols() -> list[str]:
         "symprop_tensor_save_spt",
         "symprop_gemmtn", "symprop_symgemm", "symprop_symsyrk", "symprop_qr", "symprop_syevd", "symprop_leftsvd",
         "symprop_symsyrk_device", "symprop_symgemm_device", "symprop_debug_set_tc_wait_ns",
+        "symprop_debug_set",
     ]
 
 

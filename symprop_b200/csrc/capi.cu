@@ -1,5 +1,6 @@
 // extern "C" entry points declared in include/symprop.h.  Each converts
 // C++ exceptions into status codes and keeps the last message per thread.
+#include <atomic>
 #include <cstdio>
 #include <fstream>
 #include <iomanip>
@@ -14,6 +15,8 @@ namespace spb {
 static thread_local std::string g_last_error;
 void set_last_error(const std::string &msg) { g_last_error = msg; }
 
+static std::atomic<uint64_t> g_debug[SYMPROP_DEBUG_KEYS];
+uint64_t debug_value(int key) { return g_debug[key].load(std::memory_order_relaxed); }
 
 }  // namespace spb
 
@@ -60,6 +63,13 @@ int symprop_device_count(int *count) {
 
 int symprop_set_device(int device) {
   return guard([&] { SPB_CUDA(cudaSetDevice(device)); });
+}
+
+int symprop_debug_set(int key, uint64_t value) {
+  return guard([&] {
+    require(key >= 0 && key < SYMPROP_DEBUG_KEYS, "unknown debug key");
+    g_debug[key].store(value);
+  });
 }
 
 int symprop_trim_memory(void) {

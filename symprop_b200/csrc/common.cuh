@@ -54,6 +54,9 @@ inline void cuda_check(cudaError_t e, const char *what, const char *file, int li
 #define SPB_CUDA(x) ::spb::cuda_check((x), #x, __FILE__, __LINE__)
 #define SPB_LAUNCH_CHECK() ::spb::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)
 
+// value of a SYMPROP_DEBUG_* key (capi.cu)
+uint64_t debug_value(int key);
+
 // Runs `body` and converts exceptions into a status code (C-ABI boundary).
 template <class F> int guard(F &&body) {
   try {

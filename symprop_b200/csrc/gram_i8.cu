@@ -240,6 +240,7 @@ struct I8Args {
   int ld;
   int *err;
   uint64_t wait_ns;
+  int expired_warp;           // failure injection (-1: none)
   int planes;                 // per chunk: kP of residues, one more of magnitudes
   // magnitudes: entries to be summed in FP64 go to the list
   const unsigned long long *nsq;
@@ -336,7 +337,7 @@ __global__ void __launch_bounds__(256, 1)
     if (!ok) abort_flag = 1;
   }
   __syncwarp();
-  const bool done = mbar_wait_progress(&done_bar, &progress);
+  const bool done = mbar_wait_progress(&done_bar, &progress) && warp != a.expired_warp;
   asm volatile("tcgen05.fence::after_thread_sync;");
   const int go = __all_sync(0xffffffffu, done ? 1 : 0) && !__shfl_sync(0xffffffffu, (int)abort_flag, 0);
   if (go && check) {
@@ -393,7 +394,7 @@ __global__ void __launch_bounds__(256, 1)
       d[0] = make_uint4(o[0], o[1], o[2], o[3]);
       d[1] = make_uint4(o[4], o[5], o[6], o[7]);
     }
-  } else if (threadIdx.x == 0) {
+  } else if (lane == 0) {  // every warp decides by its own clock
     atomicExch(a.err, 1);
   }
   if (threadIdx.x == 0 && (abort_flag || !done)) {
@@ -614,6 +615,7 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     a.ld = g.ld;
     a.err = err;
     a.wait_ns = mainloop_wait_ns();
+    a.expired_warp = expired_warp();
     a.planes = planes;
     a.nsq = (const unsigned long long *)nsq.p;
     a.chunk0 = c0;

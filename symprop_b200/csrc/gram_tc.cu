@@ -84,6 +84,7 @@ struct TcArgs {
   size_t split_stride;         // k blocks of split u / ntiles into C + split * split_stride
   int *err;                    // set to 1 when a wait expired
   uint64_t wait_ns;            // bound of the main-loop waits
+  int expired_warp;            // failure injection (-1: none)
 };
 
 // Shape of one operand tile in shared memory.
@@ -224,7 +225,7 @@ __global__ void __launch_bounds__(128, 1)
     if (!ok) abort_flag = 1;
   }
   __syncwarp();
-  const bool done = mbar_wait_progress(&done_bar, &progress);
+  const bool done = mbar_wait_progress(&done_bar, &progress) && warp != a.expired_warp;
   asm volatile("tcgen05.fence::after_thread_sync;");
   const int go = __all_sync(0xffffffffu, done ? 1 : 0) && !__shfl_sync(0xffffffffu, (int)abort_flag, 0) &&
                  nkb > 0;
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(128, 1)
         }
       }
     }
-  } else if (threadIdx.x == 0) {
+  } else if (lane == 0) {  // every warp decides by its own clock
     atomicExch(a.err, 1);
   }
   // teardown: the copies issued into this CTA's shared memory land before it
@@ -417,6 +418,7 @@ size_t up256(size_t x) { return (x + 255) / 256 * 256; }
 
 }  // namespace
 
+int expired_warp() { return (int)debug_value(SYMPROP_DEBUG_TC_EXPIRED_WARP) - 1; }
 uint64_t mainloop_wait_ns() { return g_mainloop_wait_ns.load(); }
 void set_mainloop_wait_ns(uint64_t ns) { g_mainloop_wait_ns.store(ns ? ns : kWaitNs); }
 
@@ -523,6 +525,7 @@ void gram(cudaStream_t st, const Split &z, bool cols_mode, double *S, void *scra
   a.split_stride = (size_t)g.dim * g.dim;
   a.err = d_err;
   a.wait_ns = mainloop_wait_ns();
+  a.expired_warp = expired_warp();
   const unsigned ctas = (unsigned)(g.ntiles * g.splits);
   if (cols_mode) {
     // operands: 64-wide column strips of H / L, kColsBK rows of k per box
@@ -586,6 +589,7 @@ void times(cudaStream_t st, const Split &z, const double *P, int r, size_t sq, s
   a.split_stride = 0;
   a.err = d_err;
   a.wait_ns = mainloop_wait_ns();
+  a.expired_warp = expired_warp();
   launch<kPanelRows, false, false, 64, kPanelStages>(st, ha, la, hb, lb, a, (unsigned)((z.rows + TM - 1) / TM));
   gather_panel_kernel<<<(unsigned)(((size_t)z.rows * r + 255) / 256), 256, 0, st>>>(Wc, z.rows, r, W, ldw);
   SPB_LAUNCH_CHECK();

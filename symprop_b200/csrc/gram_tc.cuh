@@ -52,6 +52,8 @@ void gram_split_bf16(cudaStream_t st, const float *Y, int n, int m, const float 
 // bound of the tensor-core kernels' main-loop waits (failure-injection hook)
 uint64_t mainloop_wait_ns();
 void set_mainloop_wait_ns(uint64_t ns);
+// the warp whose wait for the sums is taken as expired, -1: none (failure injection)
+int expired_warp();
 
 }  // namespace gram
 }  // namespace spb
