@@ -217,8 +217,15 @@ int symprop_symgemm_device(const float *dA, const double *dB, const double *dsca
 int symprop_debug_set_tc_wait_ns(uint64_t ns);
 /* Further failure injection for tests, for the whole process; 0 switches a key off.
  *   SYMPROP_DEBUG_TC_EXPIRED_WARP  w + 1: warp w of every tensor-core Gram CTA takes
- *                                  its wait for the sums as expired */
-enum { SYMPROP_DEBUG_TC_EXPIRED_WARP = 0, SYMPROP_DEBUG_KEYS };
+ *                                  its wait for the sums as expired
+ *   SYMPROP_DEBUG_REFUSE_COUNT     this many device allocations of at least
+ *   SYMPROP_DEBUG_REFUSE_BYTES     this many bytes are refused (both to be set) */
+enum {
+  SYMPROP_DEBUG_TC_EXPIRED_WARP = 0,
+  SYMPROP_DEBUG_REFUSE_COUNT,
+  SYMPROP_DEBUG_REFUSE_BYTES,
+  SYMPROP_DEBUG_KEYS
+};
 int symprop_debug_set(int key, uint64_t value);
 
 /* ------------------------------------------- matrix:: operations (host) */

@@ -17,6 +17,14 @@ void set_last_error(const std::string &msg) { g_last_error = msg; }
 
 static std::atomic<uint64_t> g_debug[SYMPROP_DEBUG_KEYS];
 uint64_t debug_value(int key) { return g_debug[key].load(std::memory_order_relaxed); }
+bool debug_refuses(size_t bytes) {
+  const uint64_t least = debug_value(SYMPROP_DEBUG_REFUSE_BYTES);
+  if (!least || bytes < least) return false;
+  uint64_t n = debug_value(SYMPROP_DEBUG_REFUSE_COUNT);
+  while (n && !g_debug[SYMPROP_DEBUG_REFUSE_COUNT].compare_exchange_weak(n, n - 1)) {
+  }
+  return n > 0;
+}
 
 }  // namespace spb
 

@@ -54,8 +54,9 @@ inline void cuda_check(cudaError_t e, const char *what, const char *file, int li
 #define SPB_CUDA(x) ::spb::cuda_check((x), #x, __FILE__, __LINE__)
 #define SPB_LAUNCH_CHECK() ::spb::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)
 
-// value of a SYMPROP_DEBUG_* key (capi.cu)
+// value of a SYMPROP_DEBUG_* key, and whether it refuses an allocation (capi.cu)
 uint64_t debug_value(int key);
+bool debug_refuses(size_t bytes);
 
 // Runs `body` and converts exceptions into a status code (C-ABI boundary).
 template <class F> int guard(F &&body) {
@@ -92,6 +93,24 @@ struct NvtxRange {
 cudaMemPool_t device_pool();
 void trim_pool();
 
+// cudaMalloc, or with `pool` an allocation of it on st.  A refused one is tried again
+// once the pool has given its unused memory back: it may hold what is missing.
+inline void *device_alloc(size_t bytes, cudaMemPool_t pool = nullptr, cudaStream_t st = 0) {
+  void *p = nullptr;
+  auto take = [&] {
+    if (debug_refuses(bytes)) return cudaErrorMemoryAllocation;
+    return pool ? cudaMallocFromPoolAsync(&p, bytes, pool, st) : cudaMalloc(&p, bytes);
+  };
+  cudaError_t e = take();
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    trim_pool();
+    e = take();
+  }
+  SPB_CUDA(e);
+  return p;
+}
+
 template <class T> struct DBuf {
   T *p = nullptr;
   size_t n = 0;
@@ -108,12 +127,7 @@ template <class T> struct DBuf {
   void alloc(size_t count) {
     release();
     if (count == 0) return;
-    if (cudaMalloc(&p, count * sizeof(T)) != cudaSuccess) {  // the pool may hold what is missing
-      cudaGetLastError();
-      p = nullptr;
-      trim_pool();
-      SPB_CUDA(cudaMalloc(&p, count * sizeof(T)));
-    }
+    p = static_cast<T *>(device_alloc(count * sizeof(T)));
     n = count;
   }
   // grows (never shrinks); contents are not preserved
@@ -128,7 +142,6 @@ template <class T> struct DBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
-
 // Workspace of one call on `st` from that pool, so that a repeated call waits for
 // no allocation (an FP32 Gram of 50,000 x 2,002: 1.8 to 11.8 ms with cudaMalloc
 // and cudaFree per call).  Larger ones than kPoolMax are not kept: they are
@@ -139,9 +152,7 @@ struct PoolBuf {
   cudaStream_t st;
   bool pooled = true;
   PoolBuf(size_t bytes, cudaStream_t s) : st(s), pooled(bytes <= kPoolMax) {
-    if (!bytes) return;
-    if (pooled) SPB_CUDA(cudaMallocFromPoolAsync(&p, bytes, device_pool(), st));
-    else SPB_CUDA(cudaMalloc(&p, bytes));
+    if (bytes) p = device_alloc(bytes, pooled ? device_pool() : nullptr, st);
   }
   PoolBuf(const PoolBuf &) = delete;
   PoolBuf &operator=(const PoolBuf &) = delete;

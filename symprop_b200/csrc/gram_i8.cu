@@ -52,6 +52,7 @@
 // as in gram_tc.cu.
 #include <algorithm>
 #include <cmath>
+#include <optional>
 
 #include "gram_i8.cuh"
 #include "gram_tc.cuh"
@@ -522,24 +523,6 @@ I8Plan plan_i8(int rows, int cols) {
   return g;
 }
 
-struct Pool {  // scratch from the library's stream-ordered pool
-  void *p = nullptr;
-  cudaStream_t st;
-  explicit Pool(cudaStream_t s) : st(s) {}
-  Pool(size_t bytes, cudaStream_t s) : st(s) {
-    SPB_CUDA(cudaMallocFromPoolAsync(&p, std::max<size_t>(bytes, 256), device_pool(), st));
-  }
-  bool take_operands(size_t bytes) {  // false when the device has not that much left
-    if (cudaMallocFromPoolAsync(&p, bytes, device_pool(), st) == cudaSuccess) return true;
-    cudaGetLastError();
-    p = nullptr;
-    return false;
-  }
-  ~Pool() {
-    if (p) cudaFreeAsync(p, st);
-  }
-};
-
 }  // namespace
 
 // Six launches, two waits and 256-wide tiles are paid back from about 1,500 rows
@@ -559,7 +542,7 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
                   bool componentwise) {
   const I8Plan g = plan_i8(rows, cols);
   const size_t ncs = (size_t)g.nchunk * cols;
-  Pool cmax(ncs * 8, st), sc(ncs * 4, st), flags(3 * sizeof(int), st);
+  PoolBuf cmax(ncs * 8, st), sc(ncs * 4, st), flags(3 * sizeof(int), st);
   int *bad = (int *)flags.p, *err = bad + 1;
   unsigned *npairs = (unsigned *)(bad + 2);
   SPB_CUDA(cudaMemsetAsync(cmax.p, 0, ncs * 8, st));
@@ -584,25 +567,32 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
   // 4 instead of 28 of 165 ms) and more everywhere else (29.8 instead of 28.2 ms;
   // 10,000 x 816: 0.443 instead of 0.409 ms; without a check 27.2 and 0.405 ms).
   const int planes = kP + (componentwise ? 1 : 0);
-  Pool res(st), rem(st);
-  if (!res.take_operands((size_t)g.group * planes * cols * g.kc) ||
-      !rem.take_operands((size_t)g.group * kP * g.ld * g.ld))
+  // residues, then remainders
+  const size_t res_bytes = ((size_t)g.group * planes * cols * g.kc + 255) / 256 * 256;
+  std::optional<PoolBuf> ops;
+  try {
+    ops.emplace(res_bytes + (size_t)g.group * kP * g.ld * g.ld, st);
+  } catch (const Error &e) {
+    if (e.code != SYMPROP_ERR_OOM) throw;
     return false;
-  Pool list(componentwise ? max_pairs(cols) * sizeof(int2) : 0, st), nsq(componentwise ? ncs * 8 : 0, st);
+  }
+  signed char *const res = ops->as<signed char>();
+  unsigned char *const rem = ops->as<unsigned char>() + res_bytes;
+  PoolBuf list(componentwise ? max_pairs(cols) * sizeof(int2) : 0, st), nsq(componentwise ? ncs * 8 : 0, st);
   if (componentwise) SPB_CUDA(cudaMemsetAsync(nsq.p, 0, ncs * 8, st));
   SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   for (int c0 = 0; c0 < g.nchunk; c0 += g.group) {
     const int nc = std::min(g.group, g.nchunk - c0);
     auto residues = componentwise ? residue_kernel<true> : residue_kernel<false>;
     residues<<<dim3((cols + 31) / 32, g.kc / 128, nc), 128, 0, st>>>(A, rows, cols, lda, g.chunk, g.kc,
-                                                                     (const int *)sc.p, c0, (signed char *)res.p,
+                                                                     (const int *)sc.p, c0, res,
                                                                      (unsigned long long *)nsq.p);
     SPB_LAUNCH_CHECK();
     CUtensorMap map;
     cuuint64_t dims[2] = {(cuuint64_t)g.kc, (cuuint64_t)nc * planes * cols};
     cuuint64_t strides[1] = {(cuuint64_t)g.kc};
     cuuint32_t box[2] = {kBK, kTile}, estr[2] = {1, 1};
-    const CUresult r = get_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, res.p, dims, strides, box, estr,
+    const CUresult r = get_encoder()(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, res, dims, strides, box, estr,
                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                      CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) fail(SYMPROP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
@@ -611,7 +601,7 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     a.ntile = g.ntile;
     a.ntiles = g.ntiles;
     a.kblocks = g.kc / kBK;
-    a.C = (unsigned char *)rem.p;
+    a.C = rem;
     a.ld = g.ld;
     a.err = err;
     a.wait_ns = mainloop_wait_ns();
@@ -627,7 +617,7 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     i8_gram_kernel<<<(unsigned)(g.ntiles * planes * nc), 256, kSmem, st>>>(map, a);
     SPB_LAUNCH_CHECK();
     const unsigned nt = (unsigned)((cols + 31) / 32);
-    crt_kernel<<<dim3(nt, nt), 256, 0, st>>>((const unsigned char *)rem.p, g.ld, cols, nc, c0, (const int *)sc.p,
+    crt_kernel<<<dim3(nt, nt), 256, 0, st>>>(rem, g.ld, cols, nc, c0, (const int *)sc.p,
                                              c0 > 0 ? 1 : 0, C, ldc);
     SPB_LAUNCH_CHECK();
   }
