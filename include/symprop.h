@@ -219,11 +219,14 @@ int symprop_debug_set_tc_wait_ns(uint64_t ns);
  *   SYMPROP_DEBUG_TC_EXPIRED_WARP  w + 1: warp w of every tensor-core Gram CTA takes
  *                                  its wait for the sums as expired
  *   SYMPROP_DEBUG_REFUSE_COUNT     this many device allocations of at least
- *   SYMPROP_DEBUG_REFUSE_BYTES     this many bytes are refused (both to be set) */
+ *   SYMPROP_DEBUG_REFUSE_BYTES     this many bytes are refused (both to be set)
+ *   SYMPROP_DEBUG_GRAM_CHUNKS      an FP64 Gram takes at most this many chunks of
+ *                                  rows per launch */
 enum {
   SYMPROP_DEBUG_TC_EXPIRED_WARP = 0,
   SYMPROP_DEBUG_REFUSE_COUNT,
   SYMPROP_DEBUG_REFUSE_BYTES,
+  SYMPROP_DEBUG_GRAM_CHUNKS,
   SYMPROP_DEBUG_KEYS
 };
 int symprop_debug_set(int key, uint64_t value);
@@ -347,8 +350,10 @@ int symprop_ws_predict(const symprop_tensor *t, uint32_t R, uint64_t seed, uint3
 int symprop_device_count(int *count);
 int symprop_set_device(int device);
 /* The library keeps the scratch of its dense steps (eigensolver blocks,
- * GEMM and Gram partial sums, at most about 4.5 GB of an FP64 Gram's operands) in a per-device pool between calls, so that a
- * repeated solve allocates no new scratch.  This waits for the current
+ * GEMM and Gram partial sums, the operands of the tensor-core Grams,
+ * symsyrk_device and symgemm_device) in a per-device pool between calls, so that a
+ * repeated solve allocates no new scratch: buffers of up to 4.5 GB, at most 9 GB in
+ * all; larger ones are given back when the call ends.  This waits for the current
  * device and returns the pool's unused memory to it (memory in use is not
  * touched); call it before handing the GPU to other work.  (No reference
  * counterpart: the reference allocates host memory per call.) */

@@ -1262,9 +1262,9 @@ static int top_eigs_op(cudaStream_t st, const SymApply &apply, int s, int r, dou
 }  // namespace dense
 
 // Stream-ordered scratch from a pool private to this library, one per
-// device, that keeps its memory between calls (release threshold: never):
-// the eigensolver's many small buffers cost no allocation after the first
-// iteration.  (The device's default pool releases
+// device, that keeps its memory between calls: the eigensolver's many small
+// buffers cost no allocation after the first iteration.  What it keeps is bounded
+// by two buffers of the largest size that goes there.  (The device's default pool releases
 // memory at every synchronisation unless its owner raised the threshold.)
 // symprop_trim_memory gives the unused part back, and so does a device buffer
 // whose allocation fails.
@@ -1282,7 +1282,7 @@ cudaMemPool_t device_pool() {
   props.location.id = dev;
   cudaMemPool_t pool;
   SPB_CUDA(cudaMemPoolCreate(&pool, &props));
-  uint64_t keep = ~0ull;
+  uint64_t keep = 2 * PoolBuf::kPoolMax;
   SPB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
   pools[dev] = pool;
   return pool;

@@ -64,7 +64,7 @@ namespace {
 
 constexpr int kP = 16;
 constexpr int kModulus[kP] = {256, 255, 253, 251, 247, 241, 239, 233, 229, 227, 223, 217, 211, 199, 197, 193};
-constexpr int kMaxChunk = 65536;  // rows: 2^16 * 2^106 < P / 8 and 2^16 * 2^14 = 2^30
+constexpr int kMinChunk = 1024, kMaxChunk = 65536;  // rows: 2^16 * 2^106 < P / 8 and 2^16 * 2^14 = 2^30
 constexpr int kTile = 256, kBK = 128, kNStages = 3;
 constexpr uint32_t kOperand = kTile * kBK;  // bytes
 constexpr size_t kSmem = (size_t)kNStages * 2 * kOperand + 1024;
@@ -484,27 +484,38 @@ int sms() {
 
 // Chunks of the rows.  A product takes 1024 clocks per 128 rows and about
 // 12,000 besides (loads of the first stages, reduction, tensor memory), one
-// per SM at a time: of the chunk counts the one whose waves take least, as
-// long as the chunks launched together stay within kGroupBytes.
-constexpr size_t kGroupBytes = 9ull << 29;  // 4.5 GB of residues and remainders
+// per SM at a time: of the chunk counts whose operands, chunk by chunk, take at
+// most `limit` bytes, the one whose waves take least.  `nchunk` is 0 when there is
+// none.
 struct I8Plan {
   int ntile, ntiles, ld;
-  int chunk, nchunk;  // rows per chunk
-  int kc, group;      // padded rows, chunks per launch
+  int chunk, nchunk = 0;    // rows per chunk
+  int kc, group;            // padded rows, chunks per launch
+  size_t res, bytes;        // of a launch's residues, and of all its operands
 };
 
-I8Plan plan_i8(int rows, int cols) {
+I8Plan plan_i8(int rows, int cols, int planes, size_t limit) {
   I8Plan g;
   g.ntile = (cols + kTile - 1) / kTile;
   g.ntiles = g.ntile * (g.ntile + 1) / 2;
   g.ld = g.ntile * kTile;
+  auto res = [&](int kc, int group) { return ((size_t)group * planes * cols * kc + 255) / 256 * 256; };
+  auto bytes = [&](int kc, int group) { return res(kc, group) + (size_t)group * kP * g.ld * g.ld; };
   const int n = sms();
-  const int c0 = (rows + kMaxChunk - 1) / kMaxChunk;
+  // the most rows of one chunk
+  int most = 0;
+  if (bytes(kBK, 1) <= limit) {
+    most = (int)std::min<size_t>(kMaxChunk, (limit - bytes(0, 1)) / ((size_t)planes * cols));
+    most = most / kBK * kBK;
+  }
+  if (most < std::min(rows, kMinChunk)) return g;
+  const int c0 = (rows + most - 1) / most;
+  const uint64_t cap = debug_value(SYMPROP_DEBUG_GRAM_CHUNKS);  // 0: none
   double best = 1e300;
-  for (int c = c0; c <= std::max(c0, std::min(c0 + 24, rows / 1024)); ++c) {
+  for (int c = c0; c <= std::max(c0, std::min(c0 + 24, rows / kMinChunk)); ++c) {
     const int kc = ((rows + c - 1) / c + kBK - 1) / kBK * kBK;
-    const size_t bytes = (size_t)kP * ((size_t)cols * kc + (size_t)g.ld * g.ld);
-    const int group = (int)std::max<size_t>(1, std::min<size_t>((size_t)c, kGroupBytes / bytes));
+    int group = c;
+    while (group > 1 && bytes(kc, group) > limit) --group;
     double t = 0;
     for (int x = 0; x < c; x += group) {
       const double units = (double)g.ntiles * kP * std::min(group, c - x);
@@ -512,14 +523,16 @@ I8Plan plan_i8(int rows, int cols) {
     }
     if (t < best) {
       best = t;
-      g.chunk = kc;
       g.nchunk = (rows + kc - 1) / kc;
       g.kc = kc;
       g.group = group;
     }
   }
-  g.group = std::min(g.group, g.nchunk);
   g.chunk = (rows + g.nchunk - 1) / g.nchunk;  // chunks of like length: no short last one
+  g.group = std::min(g.group, g.nchunk);
+  if (cap) g.group = (int)std::min<uint64_t>(g.group, cap);
+  g.res = res(g.kc, g.group);
+  g.bytes = bytes(g.kc, g.group);
   return g;
 }
 
@@ -540,7 +553,24 @@ static unsigned max_pairs(int cols) {
 
 bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc,
                   bool componentwise) {
-  const I8Plan g = plan_i8(rows, cols);
+  // the check of a componentwise Gram is one more plane of each chunk
+  const int planes = kP + (componentwise ? 1 : 0);
+  // operands of a launch: what the pool keeps (more, and not kept, from 16,641 columns
+  // on, where the remainders alone pass that), less when the device has not that much left
+  I8Plan g;
+  std::optional<PoolBuf> ops;
+  for (size_t limit = PoolBuf::kPoolMax; !ops; limit = g.bytes / 2) {
+    g = plan_i8(rows, cols, planes, limit);
+    if (!g.nchunk && limit == PoolBuf::kPoolMax) g = plan_i8(rows, cols, planes, 4 * limit);
+    if (!g.nchunk) return false;
+    try {
+      ops.emplace(g.bytes, st);
+    } catch (const Error &e) {
+      if (e.code != SYMPROP_ERR_OOM) throw;
+    }
+  }
+  signed char *const res = ops->as<signed char>();
+  unsigned char *const rem = ops->as<unsigned char>() + g.res;
   const size_t ncs = (size_t)g.nchunk * cols;
   PoolBuf cmax(ncs * 8, st), sc(ncs * 4, st), flags(3 * sizeof(int), st);
   int *bad = (int *)flags.p, *err = bad + 1;
@@ -566,18 +596,6 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
   // them it would cost less where the FP64 kernel has the last word (200,000 x 3,876:
   // 4 instead of 28 of 165 ms) and more everywhere else (29.8 instead of 28.2 ms;
   // 10,000 x 816: 0.443 instead of 0.409 ms; without a check 27.2 and 0.405 ms).
-  const int planes = kP + (componentwise ? 1 : 0);
-  // residues, then remainders
-  const size_t res_bytes = ((size_t)g.group * planes * cols * g.kc + 255) / 256 * 256;
-  std::optional<PoolBuf> ops;
-  try {
-    ops.emplace(res_bytes + (size_t)g.group * kP * g.ld * g.ld, st);
-  } catch (const Error &e) {
-    if (e.code != SYMPROP_ERR_OOM) throw;
-    return false;
-  }
-  signed char *const res = ops->as<signed char>();
-  unsigned char *const rem = ops->as<unsigned char>() + res_bytes;
   PoolBuf list(componentwise ? max_pairs(cols) * sizeof(int2) : 0, st), nsq(componentwise ? ncs * 8 : 0, st);
   if (componentwise) SPB_CUDA(cudaMemsetAsync(nsq.p, 0, ncs * 8, st));
   SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));

@@ -14,8 +14,8 @@ bool i8_gram_pays(int rows, int cols);
 // (columns of A).  componentwise: within rows * 2^-53 sum_k |a_ki| |a_kj| as well,
 // the bound of a sum in FP64.  False when A holds an infinity
 // or a NaN, when a componentwise Gram has many columns whose large entries lie
-// in different rows, or when there is no device memory for the operands (at
-// most about 4.5 GB, from the library's pool).  Waits for `st`,
+// in different rows, or when the device has no memory for the operands of
+// about 1,000 rows.  Of the operands the library's pool keeps at most 4.5 GB.  Waits for `st`,
 // except for the last sums of odd entries.
 bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda, double *C, int ldc,
                   bool componentwise);
