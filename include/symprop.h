@@ -221,12 +221,15 @@ int symprop_debug_set_tc_wait_ns(uint64_t ns);
  *   SYMPROP_DEBUG_REFUSE_COUNT     this many device allocations of at least
  *   SYMPROP_DEBUG_REFUSE_BYTES     this many bytes are refused (both to be set)
  *   SYMPROP_DEBUG_GRAM_CHUNKS      an FP64 Gram takes at most this many chunks of
- *                                  rows per launch */
+ *                                  rows per launch
+ *   SYMPROP_DEBUG_UNSAFE_PIVOTS    1: every unchecked restart of the eigensolver is
+ *                                  taken as numerically rank deficient */
 enum {
   SYMPROP_DEBUG_TC_EXPIRED_WARP = 0,
   SYMPROP_DEBUG_REFUSE_COUNT,
   SYMPROP_DEBUG_REFUSE_BYTES,
   SYMPROP_DEBUG_GRAM_CHUNKS,
+  SYMPROP_DEBUG_UNSAFE_PIVOTS,
   SYMPROP_DEBUG_KEYS
 };
 int symprop_debug_set(int key, uint64_t value);

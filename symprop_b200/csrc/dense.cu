@@ -1188,7 +1188,8 @@ static int top_eigs_op(cudaStream_t st, const SymApply &apply, int s, int r, dou
   // One restart from the block x: Krylov basis, Rayleigh-Ritz, the new block
   // in xn.  The quick form checks no pivot until the restart's only wait; when
   // one was not safe, the restart is done again in the careful form, which
-  // waits for each block and falls back to Householder.
+  // waits for each block and falls back to Householder, and so are the
+  // solve's other restarts.
   auto restart = [&](bool careful) {
     auto orth = [&](double *W, int j) {
       return orthonormalize(st, W, s, b, careful ? nullptr : stat.as<int>() + 2 * j);
@@ -1236,18 +1237,25 @@ static int top_eigs_op(cudaStream_t st, const SymApply &apply, int s, int r, dou
     if (!careful)
       SPB_CUDA(cudaMemcpyAsync(hstat.data(), stat.p, sizeof(int) * 2 * nblk, cudaMemcpyDeviceToHost, st));
     SPB_CUDA(cudaStreamSynchronize(st));
-    return careful || std::all_of(hstat.begin(), hstat.end(), [](int v) { return v == 0; });
+    return careful || (std::all_of(hstat.begin(), hstat.end(), [](int v) { return v == 0; }) &&
+                       !debug_value(SYMPROP_DEBUG_UNSAFE_PIVOTS));
   };
+  int repeated = 0;  // restarts done twice
+  bool careful = false;
   for (int it = 0; it <= max_restarts; ++it) {
-    if (!restart(false)) restart(true);
+    if (!careful && !restart(false)) {
+      careful = true;
+      ++repeated;
+    }
+    if (careful) restart(true);
     std::swap(x, xn);
     double scale = std::max(std::fabs(hw[0]), 1e-300);
     double worst = 0;
     for (int i = 0; i < r; ++i) worst = std::max(worst, hres[i] / scale);
     if (worst <= tol || it == max_restarts) {
       if (eig_trace())
-        std::fprintf(stderr, "top_eigs: s=%d r=%d b=%d restarts=%d residual=%.3e tol=%.1e householder=%d\n", s, r,
-                     b, it, worst, tol, g_householder_fallbacks);
+        std::fprintf(stderr, "top_eigs: s=%d r=%d b=%d restarts=%d repeated=%d residual=%.3e tol=%.1e householder=%d\n",
+                     s, r, b, it, repeated, worst, tol, g_householder_fallbacks);
       g_householder_fallbacks = 0;
       copy_cols_kernel<<<cdiv((long long)s * r, 256), 256, 0, st>>>(x, b, s, r, V, r);
       SPB_LAUNCH_CHECK();
