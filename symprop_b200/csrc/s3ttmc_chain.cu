@@ -1011,28 +1011,25 @@ ChainData &chain_data(TensorState &t) {
   cd->L = L;
   cudaStream_t st = 0;
   // degree rank of every node (0 = most frequent; ties by id)
-  DBuf<uint32_t> deg(n), key(n), key_sorted(n), ids(n), by_degree(n), rank(n);
-  SPB_CUDA(cudaMemsetAsync(deg.p, 0, sizeof(uint32_t) * n, st));
+  PoolBuf nodes(6 * sizeof(uint32_t) * (size_t)n, st);
+  uint32_t *const deg = nodes.as<uint32_t>(), *const key = deg + n, *const key_sorted = key + n,
+           *const ids = key_sorted + n, *const by_degree = ids + n, *const rank = by_degree + n;
+  SPB_CUDA(cudaMemsetAsync(deg, 0, sizeof(uint32_t) * n, st));
   if (t.nnz) {
-    degree_kernel<<<blocks_for(t.nnz * t.order, 256), 256, 0, st>>>(t.inds.p, t.nnz * t.order, deg.p);
+    degree_kernel<<<blocks_for(t.nnz * t.order, 256), 256, 0, st>>>(t.inds.p, t.nnz * t.order, deg);
     SPB_LAUNCH_CHECK();
   }
-  desc_key_kernel<<<blocks_for(n, 256), 256, 0, st>>>(deg.p, n, key.p);
+  desc_key_kernel<<<blocks_for(n, 256), 256, 0, st>>>(deg, n, key);
   SPB_LAUNCH_CHECK();
-  device_iota(ids.p, n, st);
+  device_iota(ids, n, st);
   {
     size_t tmp = 0;
-    SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, key.p, key_sorted.p, ids.p, by_degree.p, n, 0, 32, st));
-    DBuf<char> work(std::max<size_t>(tmp, 1));
-    SPB_CUDA(cub::DeviceRadixSort::SortPairs(work.p, tmp, key.p, key_sorted.p, ids.p, by_degree.p, n, 0, 32, st));
+    SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp, key, key_sorted, ids, by_degree, n, 0, 32, st));
+    PoolBuf work(std::max<size_t>(tmp, 1), st);
+    SPB_CUDA(cub::DeviceRadixSort::SortPairs(work.p, tmp, key, key_sorted, ids, by_degree, n, 0, 32, st));
   }
-  rank_kernel<<<blocks_for(n, 256), 256, 0, st>>>(by_degree.p, n, rank.p);
+  rank_kernel<<<blocks_for(n, 256), 256, 0, st>>>(by_degree, n, rank);
   SPB_LAUNCH_CHECK();
-  deg.release();
-  key.release();
-  key_sorted.release();
-  ids.release();
-  by_degree.release();
 
   // owners: leaves in pivot order; stable sort by the pivot key, then by row
   const int bits = bits_for(n ? n - 1 : 0);
@@ -1041,7 +1038,7 @@ ChainData &chain_data(TensorState &t) {
   DBuf<uint32_t> S_piv(nown * t.sstride), own_row(nown), perm_a(nown), perm_b(nown), rows_a(nown), rows_b(nown);
   DBuf<uint64_t> pkey(nown), pkey_sorted(nown);
   if (nown) {
-    pivot_order_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.own_S.p, nown, t.sstride, L, rank.p, bits, S_piv.p,
+    pivot_order_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.own_S.p, nown, t.sstride, L, rank, bits, S_piv.p,
                                                                pkey.p);
     SPB_LAUNCH_CHECK();
     owner_row_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.row_ptr.p, n, nown, own_row.p);

@@ -49,6 +49,11 @@
 // average, because closing an item (all of G through shared memory) costs as much
 // as some tens of owners (at 25 owners a node the two are equal, at 10 this one
 // takes 1.15 times as long, at 200 it is the faster one).
+//
+// The first call on a tensor also orders its owners (chain_data: two radix sorts)
+// and deals them to the warps (chain5_build); both are kept.  First call, ms, FP32,
+// R = 16, with the CTA kernel / with this one: 250 nodes, 10,000 tuples 1.00 / 0.99;
+// 20,000 nodes, 2M tuples 16.2 / 16.1; 200,000 nodes, 20M tuples 120 / 96.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -451,12 +456,12 @@ __global__ void __launch_bounds__(kThreads, CTAS) s3ttmc_group5_kernel(const Gro
 
 // Sub-groups of one item (at most 1024 owners; S in pivot order): owner i starts one when it
 // starts a group (flag bit 0, or the item's first owner) or is a multiple of
-// kSub owners into its group.  Without `first`: their number to count[item].
-// With it: the sub-groups are dealt to the building warps by size, largest
-// first (sub-group r of that stable order to warp r % 8, stage r / 8), and the
-// owners stored warp by warp in that order: S_out[k], c_out[k] are those of place
-// k, kLast set where it ends its sub-group, first[9 item + w] is warp w's first
-// place (w = 8: the item's end).
+// kSub owners into its group.  Their number goes to count[item].  They are dealt to
+// the building warps by size, largest first (sub-group r of that stable order to
+// warp r % 8, stage r / 8), and the owners stored warp by warp in that order:
+// S_out[k], c_out[k] are those of place k, kLast set where it ends its sub-group,
+// first[9 item + w] is warp w's first place (w = 8: the item's end).
+// The order is worked out in shared memory, so that the copies run along places.
 __global__ void __launch_bounds__(128) sub_groups_kernel(const Chunk *items, const uint8_t *flags, uint32_t *count,
                                                          const uint4 *S, const double *c, uint4 *S_out, double *c_out,
                                                          uint32_t *first) {
@@ -470,6 +475,7 @@ __global__ void __launch_bounds__(128) sub_groups_kernel(const Chunk *items, con
   __shared__ uint16_t starts[128 * kPer + 1];
   __shared__ uint32_t sub[128 * kPer];     // by size: start | owners << 16
   __shared__ uint16_t place[128 * kPer];   // first place of the sub-group among its warp's
+  __shared__ uint16_t from[128 * kPer];    // owner of each place, bit 15: ends its sub-group
   __shared__ uint32_t wsum[kBuildWarps];
   const Chunk ch = items[blockIdx.x];
   const int n = (int)(ch.oe - ch.ob), t = threadIdx.x;
@@ -492,10 +498,7 @@ __global__ void __launch_bounds__(128) sub_groups_kernel(const Chunk *items, con
     cnt += st[j];
   }
   Scan(tmp.scan).ExclusiveSum(cnt, rank, total);
-  if (!first) {
-    if (t == 0) count[blockIdx.x] = (uint32_t)total;
-    return;
-  }
+  if (t == 0) count[blockIdx.x] = (uint32_t)total;
 #pragma unroll
   for (int j = 0; j < kPer; ++j)
     if (st[j]) starts[rank++] = (uint16_t)(t * kPer + j);
@@ -529,15 +532,18 @@ __global__ void __launch_bounds__(128) sub_groups_kernel(const Chunk *items, con
   }
   for (int r = t; r < total; r += 128) {
     const int w = r % kBuildWarps;
-    uint32_t o = (uint32_t)ch.ob + place[r];
+    uint32_t o = place[r];
     for (int k = 0; k < w; ++k) o += wsum[k];
-    const uint32_t b = (uint32_t)ch.ob + (sub[r] & 0xffffu), len = sub[r] >> 16;
-    for (uint32_t j = 0; j < len; ++j) {
-      uint4 v = S[b + j];
-      if (j + 1 == len) v.x |= kLast;
-      S_out[o + j] = v;
-      c_out[o + j] = c[b + j];
-    }
+    const uint32_t b = sub[r] & 0xffffu, len = sub[r] >> 16;
+    for (uint32_t j = 0; j < len; ++j) from[o + j] = (uint16_t)((b + j) | (j + 1 == len ? 0x8000u : 0u));
+  }
+  __syncthreads();
+  for (int k = t; k < n; k += 128) {
+    const uint32_t f = from[k], i = f & 0x7fffu;
+    uint4 v = S[ch.ob + i];
+    if (f & 0x8000u) v.x |= kLast;
+    S_out[ch.ob + k] = v;
+    c_out[ch.ob + k] = c[ch.ob + i];
   }
 }
 
@@ -604,15 +610,14 @@ std::unique_ptr<ChainGroups> chain5_build(const TensorState &t, const ChainData 
   g->c.alloc(t.nown);
   if (!n) return g;
   cudaStream_t st = 0;
-  DBuf<Chunk> d(n);
-  DBuf<uint32_t> count(n);
-  SPB_CUDA(cudaMemcpyAsync(d.p, items.data(), n * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-  sub_groups_kernel<<<(unsigned)n, 128, 0, st>>>(d.p, cd.flags.p, count.p, nullptr, nullptr, nullptr, nullptr, nullptr);
-  SPB_LAUNCH_CHECK();
-  SPB_CUDA(cudaMemcpyAsync(g->sub.data(), count.p, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-  sub_groups_kernel<<<(unsigned)n, 128, 0, st>>>(d.p, cd.flags.p, nullptr, reinterpret_cast<const uint4 *>(cd.S.p),
+  PoolBuf tmp(n * (sizeof(Chunk) + sizeof(uint32_t)), st);
+  Chunk *const d = tmp.as<Chunk>();
+  uint32_t *const count = reinterpret_cast<uint32_t *>(d + n);
+  SPB_CUDA(cudaMemcpyAsync(d, items.data(), n * sizeof(Chunk), cudaMemcpyHostToDevice, st));
+  sub_groups_kernel<<<(unsigned)n, 128, 0, st>>>(d, cd.flags.p, count, reinterpret_cast<const uint4 *>(cd.S.p),
                                                  cd.c64.p, reinterpret_cast<uint4 *>(g->S.p), g->c.p, g->first.p);
   SPB_LAUNCH_CHECK();
+  SPB_CUDA(cudaMemcpyAsync(g->sub.data(), count, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   SPB_CUDA(cudaStreamSynchronize(st));
   return g;
 }
