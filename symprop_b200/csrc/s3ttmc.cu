@@ -473,6 +473,15 @@ void unpack_rows(const void *dpacked, uint64_t rows, uint32_t dim, uint32_t orde
   spb_check_host(st, "unpack");
 }
 
+static bool stream_capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &s) != cudaSuccess) {  // the legacy stream beside a capture of another thread
+    cudaGetLastError();
+    return false;
+  }
+  return s != cudaStreamCaptureStatusNone;
+}
+
 // A second stream of this device (created once, kept), forked from `st`
 // at construction: work queued on `side` starts after the work queued on
 // `st` so far, and join() makes later work on `st` wait for it.
@@ -517,7 +526,7 @@ struct SideFork {
 
 // One pass over a set of work items: writes the packed rows (or, when
 // `packed` is false, the full rows) [items.row0, items.row0 + items.rows) of
-// dY.  t.partials and t.scratch must already be large enough.
+// dY.  items.partials and t.scratch must already be large enough.
 static void s3ttmc_items(TensorState &t, const ItemSet &items, const void *dU, uint32_t R, bool packed,
                          void *dY, int precision, cudaStream_t st) {
   const size_t es = precision == SYMPROP_FP64 ? 8 : 4;
@@ -664,16 +673,33 @@ static bool use_chain(const TensorState &t, uint32_t R) {
   return (sched == kScheduleAuto || sched == kScheduleChain) && chain_supported(t, R);
 }
 
-static void s3ttmc_reserve(TensorState &t, uint32_t R, bool packed, int precision) {
+// The chain's work items for this call (null: another schedule) and the buffer of their partial rows.
+struct Reserved {
+  ChainItems *chain = nullptr;
+  DBuf<double> *partials = nullptr;
+};
+
+static Reserved s3ttmc_reserve(TensorState &t, uint32_t R, bool packed, int precision, bool capturing = false) {
   if (R == 0) fail(SYMPROP_ERR_INVALID, "R must be positive");
   if (precision != SYMPROP_FP64 && precision != SYMPROP_FP32)
     fail(SYMPROP_ERR_INVALID, "unknown precision %d", precision);
   const size_t es = precision == SYMPROP_FP64 ? 8 : 4;
   const uint64_t m = symsize(R, t.order - 1);
   if (!packed && t.order > 2) t.scratch.ensure((size_t)t.dim * m * es);
+  Reserved r;
+  r.partials = &t.partials;
   uint32_t slots = t.nslots;
-  if (use_chain(t, R)) slots = std::max(slots, chain_items(t, R, precision).nslots);
-  if (slots) t.partials.ensure((size_t)slots * m);
+  if (use_chain(t, R)) {
+    r.chain = &chain_items(t, R, precision, capturing);
+    if (t.order == 4 && r.chain == t.chain->items[1].get()) {
+      r.partials = &r.chain->partials;
+      slots = r.chain->nslots;
+    } else {
+      slots = std::max(slots, r.chain->nslots);
+    }
+  }
+  if (slots) r.partials->ensure((size_t)slots * m);
+  return r;
 }
 
 void s3ttmc_prepare(TensorState &t, uint32_t R, bool packed, int precision) {
@@ -683,10 +709,10 @@ void s3ttmc_prepare(TensorState &t, uint32_t R, bool packed, int precision) {
 void s3ttmc_run(TensorState &t, const void *dU, uint32_t R, bool packed, void *dY, int precision,
                 cudaStream_t st) {
   NvtxRange nv("S3TTMc");
-  s3ttmc_reserve(t, R, packed, precision);
+  const Reserved res = s3ttmc_reserve(t, R, packed, precision, stream_capturing(st));
   ItemSet all;
-  if (use_chain(t, R)) {
-    const ChainItems &cd = chain_items(t, R, precision);
+  if (res.chain) {
+    const ChainItems &cd = *res.chain;
     all.groups = cd.groups;
     all.chunks = cd.chunks.p;
     all.nchunks = cd.nchunks;
@@ -704,6 +730,7 @@ void s3ttmc_run(TensorState &t, const void *dU, uint32_t R, bool packed, void *d
     all.nsplit = t.nsplit;
     all.nslots = t.nslots;
   }
+  all.partials = res.partials->p;
   all.row0 = 0;
   all.rows = t.dim;
   s3ttmc_items(t, all, dU, R, packed, dY, precision, st);
@@ -746,7 +773,7 @@ static uint32_t host_band_count(size_t ybytes) {
 
 void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y, int precision) {
   NvtxRange nv("S3TTMc (host buffers, row bands)");
-  s3ttmc_reserve(t, R, packed, precision);
+  const Reserved res = s3ttmc_reserve(t, R, packed, precision);
   const size_t es = precision == SYMPROP_FP64 ? 8 : 4;
   uint64_t cols = packed ? symsize(R, t.order - 1) : 1;
   if (!packed)
@@ -754,8 +781,9 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
   const size_t ubytes = (size_t)t.dim * R * es, ybytes = (size_t)t.dim * cols * es;
   t.io_U.ensure(ubytes);
   t.io_Y.ensure(ybytes);
-  const bool chain = use_chain(t, R);
-  const RowBands &bd = chain ? chain_bands(t, R, precision, host_band_count(ybytes)) : row_bands(t, host_band_count(ybytes));
+  const bool chain = res.chain != nullptr;
+  const uint32_t nbands = host_band_count(ybytes);
+  const RowBands &bd = chain ? chain_bands(t, *res.chain, nbands) : row_bands(t, nbands);
 
   // SPB_TRACE_HOST=1 prints when each band's compute and copy ended
   const bool trace = std::getenv("SPB_TRACE_HOST") != nullptr;
@@ -793,8 +821,9 @@ void s3ttmc_host(TensorState &t, const void *U, uint32_t R, bool packed, void *Y
     band.row0 = bd.row0[k];
     band.rows = bd.row0[k + 1] - bd.row0[k];
     band.chain = chain;
-    band.nslots = chain ? chain_items(t, R, precision).nslots : t.nslots;
-    band.groups = chain && chain_items(t, R, precision).groups;
+    band.nslots = chain ? res.chain->nslots : t.nslots;
+    band.partials = res.partials->p;
+    band.groups = chain && res.chain->groups;
     if (!chain) band.nheavy = bd.nheavy[k];
     if (chain) {
       band.light = bd.light.p + bd.light0[k];
@@ -831,10 +860,10 @@ static void finish_rows(TensorState &t, const ItemSet &items, uint64_t m, void *
   if (items.nsplit) {
     dim3 grid(items.nsplit, (unsigned)((m + 31) / 32));
     if (precision == SYMPROP_FP64)
-      combine_kernel<double><<<grid, 256, 0, st>>>(items.split, t.partials.p, (uint32_t)m, Ypk, m, t.dim,
+      combine_kernel<double><<<grid, 256, 0, st>>>(items.split, items.partials, (uint32_t)m, Ypk, m, t.dim,
                                                    items.nslots);
     else
-      combine_kernel<float><<<grid, 256, 0, st>>>(items.split, t.partials.p, (uint32_t)m, Ypk, m, t.dim,
+      combine_kernel<float><<<grid, 256, 0, st>>>(items.split, items.partials, (uint32_t)m, Ypk, m, t.dim,
                                                   items.nslots);
     SPB_LAUNCH_CHECK();
   }

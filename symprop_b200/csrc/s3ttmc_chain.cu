@@ -476,6 +476,8 @@ template <bool MMA> constexpr int kFStride = kRP * kS2 + (MMA ? 4 : 0);
 
 struct Chain5Params {
   const Chunk *chunks;
+  const uint32_t *first;  // items of the group kernel (ChainGroups), null: ranges of owners
+  uint64_t nitems;
   uint32_t nchunks;
   const uint32_t *S;  // nown x 4 leaf ids in pivot order
   const void *c;
@@ -521,7 +523,13 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem5<T, MMA> &sm = *reinterpret_cast<Smem5<T, MMA> *>(smem_raw);
   const int tid = threadIdx.x;
-  const Chunk ch = p.chunks[blockIdx.x];
+  Chunk ch = p.chunks[blockIdx.x];
+  if (p.first) {  // an item of the group kernel: its number in ob
+    if (!SPB_BOUND(ch.ob < p.nitems, 211, blockIdx.x)) return;
+    const uint32_t *f = p.first + ch.ob * kGroupPlaces;
+    ch.ob = f[0];
+    ch.oe = f[kGroupPlaces - 1];
+  }
   if (!SPB_BOUND(ch.ob <= ch.oe && ch.oe <= p.nown && ch.row < p.nrows && (ch.slot == kDirect || ch.slot < p.nslots),
                  211, blockIdx.x))
     return;
@@ -1081,12 +1089,13 @@ ChainData &chain_data(TensorState &t) {
 // with 64.  The
 // CTA kernels lose with smaller items (R = 16, 128 instead of 256: 0.192 -> 0.215
 // ms on 10,000 nodes, 200,000 entries), their cost per item being larger.
-ChainItems &chain_items(TensorState &t, uint32_t R, int precision) {
+ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturing) {
   ChainData &cd = chain_data(t);
   const bool warp = chain8_supported(t, R);
   const bool groups = !cd.no_groups && chain5_pays(t, R, precision);
-  std::unique_ptr<ChainItems> &slot = cd.items[warp || groups];
+  std::unique_ptr<ChainItems> &slot = cd.items[warp || groups], &other = cd.items[!(warp || groups)];
   if (slot) return *slot;
+  if (other && (capturing || (t.order == 5 && !groups))) return *other;
   auto it = std::make_unique<ChainItems>();
   const uint64_t target_items = 148ull * 32ull;
   const uint64_t co = (heavy_owner_count(t) + target_items - 1) / target_items;
@@ -1101,7 +1110,7 @@ ChainItems &chain_items(TensorState &t, uint32_t R, int precision) {
     } catch (const Error &e) {  // no memory for a second copy of the owners
       if (e.code != SYMPROP_ERR_OOM) throw;
       cd.no_groups = true;
-      return chain_items(t, R, precision);
+      return chain_items(t, R, precision, capturing);
     }
   }
   sort_chain_items(cd, *it, ch, 0, ch.size());
@@ -1115,16 +1124,14 @@ ChainItems &chain_items(TensorState &t, uint32_t R, int precision) {
   return *(slot = std::move(it));
 }
 
-// (the split rows and light rows of the two order-5 kernels are the same)
 const ChainItems *built_chain_items(const TensorState &t, uint32_t R) {
   if (!t.chain) return nullptr;
   const auto &items = t.chain->items;
-  if (t.order == 5) return items[0] ? items[0].get() : items[1].get();
-  return items[chain8_supported(t, R)].get();
+  const int k = chain8_supported(t, R) ? 1 : 0;  // (order 5: both have the same split rows)
+  return items[k] ? items[k].get() : items[1 - k].get();
 }
 
-const RowBands &chain_bands(TensorState &t, uint32_t R, int precision, uint32_t nb) {
-  ChainItems &cd = chain_items(t, R, precision);
+const RowBands &chain_bands(TensorState &t, ChainItems &cd, uint32_t nb) {
   nb = std::max<uint32_t>(1, std::min<uint32_t>(nb, std::max<uint32_t>(t.dim, 1)));
   auto found = cd.bands.find(nb);
   if (found != cd.bands.end()) return *found->second;
@@ -1230,6 +1237,8 @@ void chain5_rows_launch(const TensorState &t, const ChainData &cd, const ItemSet
   const Order5Tables &tb = order5_tables(R);
   Chain5Params p;
   p.chunks = items.chunks;
+  p.first = items.groups ? cd.groups->first.p : nullptr;
+  p.nitems = items.groups ? cd.groups->sub.size() : 0;
   p.nchunks = items.nchunks;
   p.S = cd.S.p;
   p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64.p : (const void *)cd.c32.p;
@@ -1240,7 +1249,7 @@ void chain5_rows_launch(const TensorState &t, const ChainData &cd, const ItemSet
   p.m3 = (uint32_t)symsize(R, 3);
   p.m4 = (uint32_t)symsize(R, 4);
   p.Y = dYpacked;
-  p.partials = t.partials.p;
+  p.partials = items.partials;
   p.tri = tb.tri;
   p.quad = tb.quad;
   p.nown = t.nown;
@@ -1267,7 +1276,10 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
   if (!chain_supported(t, R)) fail(SYMPROP_ERR_SIZE, "chain S3TTMc does not support order %u rank %u", t.order, R);
   if (!items.nchunks) return;
   if (t.order == 5) {
-    if (items.groups) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
+    // the tables of both kernels of a rank, so that either can be captured once one has run
+    order5_tables(R);
+    chain5_tables(R);
+    if (items.groups && chain5_pays(t, R, precision)) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
     else chain5_rows_launch(t, cd, items, dU, R, dYpacked, precision, st);
     return;
   }
@@ -1287,7 +1299,7 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
   p.m2 = R * (R + 1) / 2;
   p.m3 = (uint32_t)symsize(R, 3);
   p.Y = dYpacked;
-  p.partials = t.partials.p;
+  p.partials = items.partials;
   p.trip = triples(R);
   p.nown = t.nown;
   p.nrows = t.dim;

@@ -15,10 +15,13 @@ struct ChainItems {
   DBuf<Chunk> light;              // each, for the warp-per-row kernel, heaviest first
   std::map<uint32_t, std::unique_ptr<RowBands>> bands;  // by band count
   bool groups = false;            // order 5: items of s3ttmc_chain5.cu
+  DBuf<double> partials;          // order 4, R <= 8: partial rows of its own (it has more slots, and a
+                                  // call must not move the rows of one at R > 8, captured in a graph)
 };
 
 // Order 5: the owners of every item in the order the building warps of
 // s3ttmc_chain5.cu take them.  Built on first use of a rank it covers.
+constexpr int kGroupPlaces = 9;  // of an item in `first`
 struct ChainGroups {
   DBuf<uint32_t> S;               // nown x 4 leaf ids in pivot order; bit 31 of s_1: ends its sub-group
   DBuf<double> c;                 // owner coefficients
@@ -51,19 +54,22 @@ bool chain_supported(const TensorState &t, uint32_t R);
 // The chain data of t (built on the first call).
 ChainData &chain_data(TensorState &t);
 // The work items of a rank and precision (built on first use), and in nb row bands.
-ChainItems &chain_items(TensorState &t, uint32_t R, int precision);
+// Either list of an order serves all its kernels: while a stream is captured, when
+// none can be built, the one that is there does, and at order 5 the CTA kernel takes
+// the group kernel's where there is one.
+ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturing = false);
 const ChainItems *built_chain_items(const TensorState &t, uint32_t R);  // null before the first use
-const RowBands &chain_bands(TensorState &t, uint32_t R, int precision, uint32_t nb);
+const RowBands &chain_bands(TensorState &t, ChainItems &items, uint32_t nb);
 // One pass over chain work items: packed Y rows, partial rows for split rows.
 void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
                   void *dYpacked, int precision, cudaStream_t st);
-
 
 // s3ttmc_chain5.cu (order 5): whether the group kernel is the faster one here;
 // the owners of items (ranges in row order of the owners in pivot order), dealt to
 // its warps; one pass over items whose ob is the item's number in row order and
 // whose oe - ob is its number of sub-groups.
 bool chain5_pays(const TensorState &t, uint32_t R, int precision);
+void chain5_tables(uint32_t R);  // its index table of a rank, built on first use
 std::unique_ptr<ChainGroups> chain5_build(const TensorState &t, const ChainData &cd, const std::vector<Chunk> &items);
 void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,
                    void *dYpacked, int precision, cudaStream_t st);

@@ -74,7 +74,8 @@ constexpr int kSub = 16;         // owners per sub-group
 template <typename T> constexpr int kBlk = sizeof(T) == 8 ? 2 : 4;  // owners gathered at a time by a warp
 constexpr int kStages = 2;
 constexpr uint32_t kLast = 0x80000000u;
-constexpr int kFirst = kBuildWarps + 1;  // places of an item in `first`
+constexpr int kFirst = kGroupPlaces;
+static_assert(kFirst == kBuildWarps + 1, "places of an item in `first`");
 
 // Places of T: by the middle index y, then z, then x (the lanes of a set, pairs
 // with the same y next to each other, store next to each other).
@@ -593,6 +594,8 @@ template <typename T> void dispatch(const GroupParams &p, cudaStream_t st) {
 
 }  // namespace
 
+void chain5_tables(uint32_t R) { quad_table(R); }
+
 // both sides of each line: the table above
 bool chain5_pays(const TensorState &t, uint32_t R, int precision) {
   if (t.order != 5 || !chain_supported(t, R) || t.sstride != 4) return false;
@@ -634,7 +637,7 @@ void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &ite
   p.R = R;
   p.m = (uint32_t)symsize(R, 4);
   p.Y = dYpacked;
-  p.partials = t.partials.p;
+  p.partials = items.partials;
   p.quad = quad_table(R);
   p.nentries = cd.groups->sub.size() + 1024;  // item number + sub-groups
   p.nown = t.nown;

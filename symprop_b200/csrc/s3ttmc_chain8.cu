@@ -349,7 +349,7 @@ void chain8_launch(const TensorState &t, const ChainData &cd, const ItemSet &ite
   p.R = R;
   p.m3 = (uint32_t)symsize(R, 3);
   p.Y = dYpacked;
-  p.partials = t.partials.p;
+  p.partials = items.partials;
   p.trip = triples8(R);
   p.nown = t.nown;
   p.nrows = t.dim;

@@ -74,6 +74,7 @@ struct ItemSet {
   bool chain = false;      // items of the pivot-chain schedule (ChainData)
   bool groups = false;     // of its order-5 group kernel (ChainGroups)
   uint32_t nslots = 0;     // partial-sum slots of the item list
+  double *partials = nullptr;  // and their rows
   const Chunk *light = nullptr;  // chain schedule: light rows, one chunk each
   uint32_t nlight = 0;
 };
