@@ -482,25 +482,25 @@ static bool stream_capturing(cudaStream_t st) {
   return s != cudaStreamCaptureStatusNone;
 }
 
-// A second stream of this device (created once, kept), forked from `st`
-// at construction: work queued on `side` starts after the work queued on
-// `st` so far, and join() makes later work on `st` wait for it.
+// A second stream of this device (created once, kept; one for each `kind` of
+// call), forked from `st` at construction: work queued on `side` starts after the
+// work queued on `st` so far, and join() makes later work on `st` wait for it.
 struct SideFork {
   cudaStream_t st, side;
   cudaEvent_t forked = nullptr, done = nullptr;
   bool joined = false;
-  explicit SideFork(cudaStream_t s) : st(s) {
+  SideFork(cudaStream_t s, int kind) : st(s) {
     static std::mutex mu;
-    static std::map<int, cudaStream_t> sides;
+    static std::map<std::pair<int, int>, cudaStream_t> sides;
     int dev = 0;
     SPB_CUDA(cudaGetDevice(&dev));
     {
       std::lock_guard<std::mutex> lock(mu);
-      auto it = sides.find(dev);
+      auto it = sides.find({dev, kind});
       if (it == sides.end()) {
         cudaStream_t x;
         SPB_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-        it = sides.emplace(dev, x).first;
+        it = sides.emplace(std::make_pair(dev, kind), x).first;
       }
       side = it->second;
     }
@@ -559,7 +559,7 @@ static void s3ttmc_items(TensorState &t, const ItemSet &items, const void *dU, u
         // the two kernels write disjoint rows: the light rows run on a side
         // stream, forked from and joined back into `st`, beside the chain
         // kernel (which leaves most issue slots idle)
-        SideFork fork(st);
+        SideFork fork(st, 0);
         warp_launch(*it->second, t, light, dU, Ypk, precision, fork.side);
         chain_launch(t, *t.chain, items, dU, R, Ypk, precision, st);
         fork.join();
@@ -577,8 +577,9 @@ static void s3ttmc_items(TensorState &t, const ItemSet &items, const void *dU, u
   if (sched == kScheduleAuto && split_supported(t.order, R)) {
     auto it = t.split_plans.find(R);
     if (it == t.split_plans.end()) it = t.split_plans.emplace(R, split_plan(t.order, R)).first;
-    // small ranks: the light rows on the warp-per-row kernel (disjoint rows,
-    // on a side stream when there are rows of both kinds)
+    // small ranks: the light rows on the warp-per-row kernel (disjoint rows, on a
+    // side stream when there are rows of both kinds; not in a capture, which
+    // would keep that stream from the calls of other streams and threads)
     ItemSet heavy = items, light = items;
     if (const uint32_t nh = split_heavy(R, items); nh < items.nchunks) {
       heavy.nchunks = nh;
@@ -586,12 +587,13 @@ static void s3ttmc_items(TensorState &t, const ItemSet &items, const void *dU, u
       light.nchunks -= nh;
       auto wt = t.warp.find(R);
       if (wt == t.warp.end()) wt = t.warp.emplace(R, warp_plan(t.order, R)).first;
-      if (nh) {
-        SideFork fork(st);
+      if (nh && !stream_capturing(st)) {
+        SideFork fork(st, 1);
         warp_launch(*wt->second, t, light, dU, Ypk, precision, fork.side);
         split_launch(*it->second, t, heavy, dU, Ypk, precision, st);
         fork.join();
       } else {
+        if (nh) split_launch(*it->second, t, heavy, dU, Ypk, precision, st);
         warp_launch(*wt->second, t, light, dU, Ypk, precision, st);
       }
     } else {

@@ -90,3 +90,20 @@ def test_order4_graph_outlives_a_call_at_a_smaller_rank(gpu):
     g.replay()
     c.check(t, v)
     assert torch.isnan(fill).all()
+
+
+@pytest.mark.parametrize("R,prec", [(8, "f64"), (5, "f32"), (10, "f32")])
+def test_order6(gpu, R, prec):
+    """Rows of both kinds (at most 8 owners, more); a capture keeps no stream from other calls."""
+    import torch
+    X, t, v = tensor(gpu, 6, 400, 900, s=1.1, seed=6)
+    X2, t2, v2 = tensor(gpu, 6, 300, 800, s=1.1, seed=7)
+    c, o = Call(gpu, X, R, prec).eager(), Call(gpu, X2, R, prec).eager()
+    g, s, s2 = torch.cuda.CUDAGraph(), torch.cuda.Stream(), torch.cuda.Stream()
+    with torch.cuda.graph(g, stream=s, capture_error_mode="relaxed"):
+        c.run(s.cuda_stream)
+        o.run(s2.cuda_stream)
+    c.Y.fill_(float("nan"))
+    g.replay()
+    c.check(t, v)
+    o.check(t2, v2)
