@@ -210,9 +210,9 @@ __global__ void __launch_bounds__(kThreads, CTAS) s3ttmc_group5_kernel(const Gro
           const int q0 = q & 15, q1 = (q >> 4) & 15, q2 = (q >> 8) & 15, q3 = q >> 12;
           const int2 f1 = sF[q1], f2 = sF[q2];
           const int z1 = f1.x + q0, z2 = f2.x + q3 * f2.y;
-          const T y = sG[q0 * G::ldG + z2 + q1] + sG[q1 * G::ldG + z2 + q0] + sG[q2 * G::ldG + z1 + q3 * f1.y] +
-                      sG[q3 * G::ldG + z1 + q2 * f1.y];
-          put<T>(p, w.row, w.slot, e, (double)y);
+          const double y = (double)sG[q0 * G::ldG + z2 + q1] + (double)sG[q1 * G::ldG + z2 + q0] +
+                           (double)sG[q2 * G::ldG + z1 + q3 * f1.y] + (double)sG[q3 * G::ldG + z1 + q2 * f1.y];
+          put<T>(p, w.row, w.slot, e, y);
         }
         bar_sync<kMul>(kBarMul);
       }
