@@ -112,6 +112,14 @@ __global__ void __launch_bounds__(128) col_max_kernel(const double *__restrict__
   atomicMax(&cmax[(size_t)blockIdx.y * cols + c], m);
 }
 
+// Entries of a componentwise Gram that have to be summed in FP64.  Past the limit
+// the FP64 kernel does all of them, and what is still queued returns at once.
+struct Odd {
+  int2 *pairs;
+  unsigned *count, max;
+  __device__ __forceinline__ bool too_many() const { return *(volatile unsigned *)count > max; }
+};
+
 // Exponent s of every column: |a| 2^s < 2^53; *bad is set when one is not finite
 __global__ void scale_kernel(const unsigned long long *cmax, int n, int *s, int *bad) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -135,7 +143,8 @@ template <bool MAG>
 __global__ void __launch_bounds__(128) residue_kernel(const double *__restrict__ A, int rows, int cols, int lda,
                                                       int chunk, int kc, const int *__restrict__ s, int chunk0,
                                                       signed char *__restrict__ out,
-                                                      unsigned long long *__restrict__ nsq) {
+                                                      unsigned long long *__restrict__ nsq, const Odd odd) {
+  if (odd.too_many()) return;
   constexpr int kPlanes = kP + (MAG ? 1 : 0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
   const int k0 = blockIdx.y * 128 + warp * 32;  // within the chunk
@@ -243,11 +252,11 @@ struct I8Args {
   uint64_t wait_ns;
   int expired_warp;           // failure injection (-1: none)
   int planes;                 // per chunk: kP of residues, one more of magnitudes
+  int nchunk;                 // of this launch
   // magnitudes: entries to be summed in FP64 go to the list
   const unsigned long long *nsq;
   int chunk0, chunk, rows;
-  int2 *pairs;
-  unsigned *npairs, max_pairs;
+  Odd odd;
 };
 
 __global__ void __launch_bounds__(256, 1)
@@ -260,9 +269,12 @@ __global__ void __launch_bounds__(256, 1)
   __shared__ volatile int progress;
   __shared__ int issued[kNStages];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // unit: tile fastest, so that the CTAs of a wave share a modulus in L2
-  const int plane = (int)blockIdx.x / a.ntiles;
-  int ti = 0, tj = (int)blockIdx.x - plane * a.ntiles;
+  // unit: tile fastest, so that the CTAs of a wave share a modulus in L2; the
+  // magnitudes of all chunks first
+  const int unit = (int)blockIdx.x / a.ntiles, checks = (a.planes - kP) * a.nchunk, residues = unit - checks;
+  const int plane = residues < 0 ? unit * a.planes + kP : residues / kP * a.planes + residues % kP;
+  if (checks && __syncthreads_or(threadIdx.x == 0 && a.odd.too_many())) return;
+  int ti = 0, tj = (int)blockIdx.x - unit * a.ntiles;
   while (tj >= a.ntile - ti) {
     tj -= a.ntile - ti;
     ++ti;
@@ -356,9 +368,9 @@ __global__ void __launch_bounds__(256, 1)
         const int j = tj * kTile + c + q;
         if (ni > 0.f && nj > 0.f && i <= j && !(ni + nj <= unit * (float)(int)v[q])) {
           // past the limit the count no longer matters (and may not wrap)
-          if (*(volatile unsigned *)a.npairs > a.max_pairs) continue;
-          const unsigned at = atomicAdd(a.npairs, 1u);
-          if (at < a.max_pairs) a.pairs[at] = make_int2(i, j);
+          if (a.odd.too_many()) continue;
+          const unsigned at = atomicAdd(a.odd.count, 1u);
+          if (at < a.odd.max) a.odd.pairs[at] = make_int2(i, j);
         }
       }
     }
@@ -423,8 +435,8 @@ __global__ void __launch_bounds__(256, 1)
 // rounding is never in doubt), scaled back and added in FP64, chunks in order.
 __global__ void __launch_bounds__(256) crt_kernel(const unsigned char *__restrict__ R, int ld, int cols, int nchunk,
                                                   int chunk0, const int *__restrict__ s, int add,
-                                                  double *__restrict__ C, int ldc) {
-  if (blockIdx.x < blockIdx.y) return;
+                                                  double *__restrict__ C, int ldc, const Odd odd) {
+  if (blockIdx.x < blockIdx.y || odd.too_many()) return;
   __shared__ double t[32][33];
   const int j0 = blockIdx.x * 32, i0 = blockIdx.y * 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const size_t pl = (size_t)ld * ld;
@@ -574,7 +586,6 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
   const size_t ncs = (size_t)g.nchunk * cols;
   PoolBuf cmax(ncs * 8, st), sc(ncs * 4, st), flags(3 * sizeof(int), st);
   int *bad = (int *)flags.p, *err = bad + 1;
-  unsigned *npairs = (unsigned *)(bad + 2);
   SPB_CUDA(cudaMemsetAsync(cmax.p, 0, ncs * 8, st));
   SPB_CUDA(cudaMemsetAsync(flags.p, 0, 3 * sizeof(int), st));
   const int part = 512;
@@ -592,11 +603,11 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     return !h[0] && (unsigned)h[2] <= max_pairs(cols);
   };
   if (!read_flags()) return false;
-  // The check of a componentwise Gram runs with the residues and their product.  Before
-  // them it would cost less where the FP64 kernel has the last word (200,000 x 3,876:
-  // 4 instead of 28 of 165 ms) and more everywhere else (29.8 instead of 28.2 ms;
-  // 10,000 x 816: 0.443 instead of 0.409 ms; without a check 27.2 and 0.405 ms).
+  // The check of a componentwise Gram runs with the residues and their product.  By
+  // itself before them it would cost more where it passes (200,000 x 3,876: 29.8 instead
+  // of 28.2 ms; 10,000 x 816: 0.443 instead of 0.409 ms; without a check 27.2 and 0.405).
   PoolBuf list(componentwise ? max_pairs(cols) * sizeof(int2) : 0, st), nsq(componentwise ? ncs * 8 : 0, st);
+  const Odd odd{list.as<int2>(), (unsigned *)(bad + 2), max_pairs(cols)};
   if (componentwise) SPB_CUDA(cudaMemsetAsync(nsq.p, 0, ncs * 8, st));
   SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   for (int c0 = 0; c0 < g.nchunk; c0 += g.group) {
@@ -604,7 +615,7 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     auto residues = componentwise ? residue_kernel<true> : residue_kernel<false>;
     residues<<<dim3((cols + 31) / 32, g.kc / 128, nc), 128, 0, st>>>(A, rows, cols, lda, g.chunk, g.kc,
                                                                      (const int *)sc.p, c0, res,
-                                                                     (unsigned long long *)nsq.p);
+                                                                     (unsigned long long *)nsq.p, odd);
     SPB_LAUNCH_CHECK();
     CUtensorMap map;
     cuuint64_t dims[2] = {(cuuint64_t)g.kc, (cuuint64_t)nc * planes * cols};
@@ -625,23 +636,22 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     a.wait_ns = mainloop_wait_ns();
     a.expired_warp = expired_warp();
     a.planes = planes;
+    a.nchunk = nc;
     a.nsq = (const unsigned long long *)nsq.p;
     a.chunk0 = c0;
     a.chunk = g.chunk;
     a.rows = rows;
-    a.pairs = (int2 *)list.p;
-    a.npairs = npairs;
-    a.max_pairs = max_pairs(cols);
+    a.odd = odd;
     i8_gram_kernel<<<(unsigned)(g.ntiles * planes * nc), 256, kSmem, st>>>(map, a);
     SPB_LAUNCH_CHECK();
     const unsigned nt = (unsigned)((cols + 31) / 32);
     crt_kernel<<<dim3(nt, nt), 256, 0, st>>>(rem, g.ld, cols, nc, c0, (const int *)sc.p,
-                                             c0 > 0 ? 1 : 0, C, ldc);
+                                             c0 > 0 ? 1 : 0, C, ldc, odd);
     SPB_LAUNCH_CHECK();
   }
   if (!read_flags()) return false;
-  if (const unsigned odd = (unsigned)h[2]) {
-    pair_kernel<<<odd, 256, 0, st>>>((const int2 *)list.p, A, rows, lda, C, ldc);
+  if (h[2]) {
+    pair_kernel<<<(unsigned)h[2], 256, 0, st>>>(odd.pairs, A, rows, lda, C, ldc);
     SPB_LAUNCH_CHECK();
   }
   return true;
