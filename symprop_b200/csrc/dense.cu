@@ -858,28 +858,46 @@ __global__ void core_reduce_kernel(const double *__restrict__ P, int chunks, int
 
 // ------------------------------------------------------------ public API
 
-// C = A^T A (upper tiles computed, the rest mirrored) for a row-major
-// K x M matrix A; M even, lda even, A 16-byte aligned.
-static void gram_f64(cudaStream_t st, int M, int K, const double *A, int lda, double *C, int ldc) {
+// Tiles and K splits of gram_f64: the fewest splits (each at least 1024 rows)
+// that fill 90% of the waves of one CTA per SM.
+struct GramSplits {
+  int nt, splits, kchunk;
+  long long tiles, waves;
+};
+
+static GramSplits gram_splits(int M, int K) {
   static int nsm = 0;
   if (!nsm) {
     int dev = 0;
     SPB_CUDA(cudaGetDevice(&dev));
     SPB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   }
-  const int nt = (M + GB - 1) / GB;
-  const long long tiles = (long long)nt * (nt + 1) / 2;
-  // the fewest K splits (each at least 1024 rows) that fill 90% of the
-  // waves of one CTA per SM
-  int splits = 1;
+  GramSplits g;
+  g.nt = (M + GB - 1) / GB;
+  g.tiles = (long long)g.nt * (g.nt + 1) / 2;
+  g.splits = 1;
   for (int s = 1; s <= 8; ++s) {
     if (s > 1 && K / s < 1024) break;
-    const long long ctas = tiles * s, waves = (ctas + nsm - 1) / nsm;
-    splits = s;
+    const long long ctas = g.tiles * s, waves = (ctas + nsm - 1) / nsm;
+    g.splits = s;
     if ((double)ctas >= 0.9 * (double)(waves * nsm)) break;
   }
-  const int kchunk = (int)(cdiv(cdiv(K, splits), GK) * GK);
-  splits = std::max(1, (int)cdiv(K, kchunk));
+  g.kchunk = (int)(cdiv(cdiv(K, g.splits), GK) * GK);
+  g.splits = std::max(1, (int)cdiv(K, g.kchunk));
+  g.waves = (g.tiles * g.splits + nsm - 1) / nsm;
+  return g;
+}
+
+static bool gram_f64_takes(int M, const double *A, int lda) {
+  return M >= GB && M % 2 == 0 && lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0;
+}
+
+// C = A^T A (upper tiles computed, the rest mirrored) for a row-major
+// K x M matrix A; M even, lda even, A 16-byte aligned.
+static void gram_f64(cudaStream_t st, int M, int K, const double *A, int lda, double *C, int ldc) {
+  const GramSplits g = gram_splits(M, K);
+  const int nt = g.nt, splits = g.splits, kchunk = g.kchunk;
+  const long long tiles = g.tiles;
   Scratch ws(sizeof(double) * (size_t)splits * M * M, st);
   const size_t smem = sizeof(GramSmem);
   SPB_CUDA(cudaFuncSetAttribute(gram_tn_f64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -908,8 +926,8 @@ void gemm(cudaStream_t st, int M, int N, int K, T alpha, const T *A, int lda, bo
       SPB_LAUNCH_CHECK();
       return;
     }
-    if (transA && !transB && sym_upper && A == B && lda == ldb && M == N && !kscale && M >= GB && M % 2 == 0 &&
-        lda % 2 == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0 && alpha == 1.0 && beta == 0.0) {
+    if (transA && !transB && sym_upper && A == B && lda == ldb && M == N && !kscale && gram_f64_takes(M, A, lda) &&
+        alpha == 1.0 && beta == 0.0) {
       gram_f64(st, M, K, A, lda, C, ldc);
       return;
     }
@@ -1009,8 +1027,21 @@ void householder_q(cudaStream_t st, double *A, int rows, int cols) {
   SPB_CUDA(cudaMemcpyAsync(A, Q.p, sizeof(double) * (size_t)rows * cols, cudaMemcpyDeviceToDevice, st));
 }
 
+// Time of the FP64 column Gram in us (within 15% over 1,536 to 80,000 rows and 320 to
+// 2,002 columns): gram_f64 takes 0.2 us a row and wave, the 64-wide tiles of
+// gemm 4e6 FMAs a us.
+static double f64_gram_us(const double *A, int rows, int cols) {
+  if (gram_f64_takes(cols, A, cols)) {
+    const GramSplits g = gram_splits(cols, rows);
+    return 25.0 + 0.2 * (double)g.kchunk * (double)g.waves;
+  }
+  const double nt = cdiv(cols, 64);
+  return 30.0 + nt * (nt + 1) / 2 * 4096.0 * rows / 4e6;
+}
+
 void gram_cols(cudaStream_t st, const double *A, int rows, int cols, double *C, GramUse use) {
-  if (gram::i8_gram_pays(rows, cols) && gram::gram_cols_i8(st, A, rows, cols, cols, C, cols, use == GramUse::kEntries))
+  if (gram::i8_gram_takes(rows, cols) && gram::i8_gram_us(rows, cols) <= f64_gram_us(A, rows, cols) &&
+      gram::gram_cols_i8(st, A, rows, cols, cols, C, cols, use == GramUse::kEntries))
     return;
   gemm<double>(st, cols, cols, rows, 1.0, A, cols, true, A, cols, false, 0.0, C, cols, nullptr, true);
 }

@@ -496,7 +496,8 @@ int sms() {
 
 // Chunks of the rows.  A product takes 1024 clocks per 128 rows and about
 // 12,000 besides (loads of the first stages, reduction, tensor memory), one
-// per SM at a time: of the chunk counts whose operands, chunk by chunk, take at
+// per SM at a time; the remainders of a chunk are put together in 18 us at 320 columns
+// (latency) and 75 us at 2,002: of the chunk counts whose operands, chunk by chunk, take at
 // most `limit` bytes, the one whose waves take least.  `nchunk` is 0 when there is
 // none.
 struct I8Plan {
@@ -528,9 +529,9 @@ I8Plan plan_i8(int rows, int cols, int planes, size_t limit) {
     const int kc = ((rows + c - 1) / c + kBK - 1) / kBK * kBK;
     int group = c;
     while (group > 1 && bytes(kc, group) > limit) --group;
-    double t = 0;
+    double t = c * std::max(35000.0, 0.035 * cols * cols);
     for (int x = 0; x < c; x += group) {
-      const double units = (double)g.ntiles * kP * std::min(group, c - x);
+      const double units = (double)g.ntiles * planes * std::min(group, c - x);
       t += std::ceil(units / n) * (kc / kBK * 1024.0 + 12000.0);
     }
     if (t < best) {
@@ -550,11 +551,20 @@ I8Plan plan_i8(int rows, int cols, int planes, size_t limit) {
 
 }  // namespace
 
-// Six launches, two waits and 256-wide tiles are paid back from about 1,500 rows
-// on (2,000 x 816: 0.43 -> 0.19 ms, 2,000 x 3,876: 1.73 -> 1.01 ms; 1,024 x
-// 2,002: 0.27 -> 0.31 ms) and from about 320 columns (10,000 x 256: 0.28 ms
-// either way).
-bool i8_gram_pays(int rows, int cols) { return cols >= 320 && rows >= 1536; }
+// Six launches, two waits and 256-wide tiles take 130 us and more, so that the FP64
+// kernels win where they are not at their own worst: us, FP64 kernel / this one:
+//   rows                     1,536      3,000      6,000      10,000     40,000
+//   320 columns (even)     336 / 146  329 / 155  270 / 178  286 / 246  1,025 / 413
+//   321 (odd, gemm)         66 / 144   96 / 153  173 / 168  254 / 244    983 / 403
+//   513                    109 / 153  180 / 161  324 / 234  516 / 281  2,057 / 552
+//   816                    338 / 172  335 / 230  280 / 304  439 / 367  1,628 / 803
+//   2,002                  365 / 376  662 / 448  1,261 / 566  2,059 / 716  8,048 / 2,018
+// The caller compares the two times (f64_gram_us in dense.cu).  This one is fitted to
+// where they meet, over 190 sizes of 1,536 to 80,000 rows and 320 to 2,002 columns: the
+// slower kernel is taken at five of them, and then by at most 10%.  Not below 320
+// columns or 1,536 rows, where it was not measured to win.
+bool i8_gram_takes(int rows, int cols) { return cols >= 320 && rows >= 1536; }
+double i8_gram_us(int rows, int cols) { return 80.0 + 0.01 * rows + 0.04 * cols + 1e-5 * rows * cols; }
 
 // Entries that the caller of a componentwise Gram may have summed one by one: 64
 // bytes of A a row each, against cols^2 / 2 FMAs a row for all of them by the FP64

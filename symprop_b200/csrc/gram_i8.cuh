@@ -6,9 +6,10 @@
 namespace spb {
 namespace gram {
 
-// Whether the column Gram of a rows x cols FP64 matrix goes to the integer
-// tensor cores.
-bool i8_gram_pays(int rows, int cols);
+// Whether gram_cols_i8 is for the column Gram of a rows x cols FP64 matrix, and about
+// how long it takes (us).
+bool i8_gram_takes(int rows, int cols);
+double i8_gram_us(int rows, int cols);
 // C (cols x cols, full symmetric, row stride ldc) = A^T A for a row-major
 // rows x cols FP64 A (row stride lda), each entry within about 2^-53 |a_i| |a_j|
 // (columns of A).  componentwise: within rows * 2^-53 sum_k |a_ki| |a_kj| as well,
