@@ -151,7 +151,7 @@ struct PoolBuf {
   void *p = nullptr;
   cudaStream_t st;
   bool pooled = true;
-  PoolBuf(size_t bytes, cudaStream_t s) : st(s), pooled(bytes <= kPoolMax) {
+  PoolBuf(size_t bytes, cudaStream_t s, size_t most = kPoolMax) : st(s), pooled(bytes <= most) {
     if (bytes) p = device_alloc(bytes, pooled ? device_pool() : nullptr, st);
   }
   PoolBuf(const PoolBuf &) = delete;

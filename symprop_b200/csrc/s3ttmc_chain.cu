@@ -1043,26 +1043,38 @@ ChainData &chain_data(TensorState &t) {
   const int bits = bits_for(n ? n - 1 : 0);
   const int key_bits = bits * (int)(L - 1);
   if (key_bits > 64) fail(SYMPROP_ERR_SIZE, "chain schedule: pivot key of %d bits", key_bits);
-  DBuf<uint32_t> S_piv(nown * t.sstride), own_row(nown), perm_a(nown), perm_b(nown), rows_a(nown), rows_b(nown);
-  DBuf<uint64_t> pkey(nown), pkey_sorted(nown);
+  // Temporaries in one buffer, of the pool up to 256 MB: nine allocations and frees of
+  // their own took two thirds of a first call (6 of 8.3 ms at 1M owners).
+  size_t tmp1 = 0, tmp2 = 0, used = 0;
+  using U32 = uint32_t *;
+  using U64 = uint64_t *;
+  SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp1, U64(), U64(), U32(), U32(), nown, 0, std::max(key_bits, 1), st));
+  SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp2, U32(), U32(), U32(), U32(), nown, 0, bits_for(n), st));
+  auto place = [&](size_t bytes) {
+    const size_t at = used;
+    used += (bytes + 255) / 256 * 256;
+    return at;
+  };
+  const size_t work_bytes = std::max(tmp1, tmp2), at_work = place(work_bytes), at_S = place(4 * nown * t.sstride),
+               at_row = place(4 * nown), at_pa = place(4 * nown), at_pb = place(4 * nown), at_ra = place(4 * nown),
+               at_rb = place(4 * nown), at_k = place(8 * nown), at_ks = place(8 * nown);
+  PoolBuf tmp(used, st, size_t(256) << 20);
+  char *const base = tmp.as<char>();
+  const U32 S_piv = U32(base + at_S), own_row = U32(base + at_row), perm_a = U32(base + at_pa),
+            perm_b = U32(base + at_pb), rows_a = U32(base + at_ra), rows_b = U32(base + at_rb);
+  const U64 pkey = U64(base + at_k), pkey_sorted = U64(base + at_ks);
   if (nown) {
-    pivot_order_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.own_S.p, nown, t.sstride, L, rank, bits, S_piv.p,
-                                                               pkey.p);
+    pivot_order_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.own_S.p, nown, t.sstride, L, rank, bits, S_piv, pkey);
     SPB_LAUNCH_CHECK();
-    owner_row_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.row_ptr.p, n, nown, own_row.p);
+    owner_row_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.row_ptr.p, n, nown, own_row);
     SPB_LAUNCH_CHECK();
-    device_iota(perm_a.p, nown, st);
-    size_t tmp1 = 0, tmp2 = 0;
-    SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp1, pkey.p, pkey_sorted.p, perm_a.p, perm_b.p, nown, 0,
+    device_iota(perm_a, nown, st);
+    size_t bytes = work_bytes;
+    SPB_CUDA(cub::DeviceRadixSort::SortPairs(base + at_work, bytes, pkey, pkey_sorted, perm_a, perm_b, nown, 0,
                                              std::max(key_bits, 1), st));
-    SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp2, rows_a.p, rows_b.p, perm_b.p, perm_a.p, nown, 0,
-                                             bits_for(n), st));
-    DBuf<char> work(std::max<size_t>(std::max(tmp1, tmp2), 1));
-    SPB_CUDA(cub::DeviceRadixSort::SortPairs(work.p, tmp1, pkey.p, pkey_sorted.p, perm_a.p, perm_b.p, nown, 0,
-                                             std::max(key_bits, 1), st));
-    gather_rows_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_b.p, own_row.p, nown, rows_a.p);
+    gather_rows_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_b, own_row, nown, rows_a);
     SPB_LAUNCH_CHECK();
-    SPB_CUDA(cub::DeviceRadixSort::SortPairs(work.p, tmp2, rows_a.p, rows_b.p, perm_b.p, perm_a.p, nown, 0,
+    SPB_CUDA(cub::DeviceRadixSort::SortPairs(base + at_work, bytes, rows_a, rows_b, perm_b, perm_a, nown, 0,
                                              bits_for(n), st));
   }
   cd->S.alloc(nown * t.sstride);
@@ -1070,10 +1082,10 @@ ChainData &chain_data(TensorState &t) {
   cd->c32.alloc(nown);
   cd->flags.alloc(nown);
   if (nown) {
-    chain_gather_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_a.p, nown, t.sstride, S_piv.p, t.own_c64.p, cd->S.p,
+    chain_gather_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_a, nown, t.sstride, S_piv, t.own_c64.p, cd->S.p,
                                                                cd->c64.p, cd->c32.p);
     SPB_LAUNCH_CHECK();
-    chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S.p, rows_b.p, nown, t.sstride, L, cd->flags.p);
+    chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S.p, rows_b, nown, t.sstride, L, cd->flags.p);
     SPB_LAUNCH_CHECK();
   }
   SPB_CUDA(cudaDeviceSynchronize());

@@ -52,8 +52,8 @@
 //
 // The first call on a tensor also orders its owners (chain_data: two radix sorts)
 // and deals them to the warps (chain5_build); both are kept.  First call, ms, FP32,
-// R = 16, with the CTA kernel / with this one: 250 nodes, 10,000 tuples 1.00 / 0.99;
-// 20,000 nodes, 2M tuples 16.2 / 16.1; 200,000 nodes, 20M tuples 120 / 96.
+// before this kernel / now: 250 nodes, 10,000 tuples, R = 8 1.02 / 0.92; 20,000 nodes,
+// 2M tuples, R = 16 16.7 / 10.4; 200,000 nodes, 20M tuples 127 / 95.
 #include <cub/cub.cuh>
 
 #include <algorithm>
