@@ -924,13 +924,14 @@ __global__ void chain_gather_kernel(const uint32_t *perm, uint64_t nown, uint32_
   c32[o] = (float)c_in[src];
 }
 
-// bit k: owner o starts a new prefix of k + 1 pivots (a new row starts all)
+// bit k: owner o starts a new prefix of k + 1 pivots (a new row starts all);
+// *ngroups: how many have bit 0
 __global__ void chain_flags_kernel(const uint32_t *S, const uint32_t *row_sorted, uint64_t nown, uint32_t sstride,
-                                   uint32_t L, uint8_t *flags) {
+                                   uint32_t L, uint8_t *flags, unsigned long long *ngroups) {
   const uint64_t o = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= nown) return;
   uint32_t f = 0;
-  if (o == 0 || row_sorted[o] != row_sorted[o - 1]) {
+  if (o >= nown) {
+  } else if (o == 0 || row_sorted[o] != row_sorted[o - 1]) {
     f = 0xffu;
   } else {
     bool differ = false;
@@ -939,7 +940,9 @@ __global__ void chain_flags_kernel(const uint32_t *S, const uint32_t *row_sorted
       if (differ) f |= 1u << k;
     }
   }
-  flags[o] = (uint8_t)f;
+  if (o < nown) flags[o] = (uint8_t)f;
+  const int groups = __syncthreads_count((int)(f & 1u));
+  if (threadIdx.x == 0 && groups) atomicAdd(ngroups, (unsigned long long)groups);
 }
 
 inline unsigned blocks_for(uint64_t n, unsigned b) { return (unsigned)std::max<uint64_t>(1, (n + b - 1) / b); }
@@ -1057,7 +1060,7 @@ ChainData &chain_data(TensorState &t) {
   };
   const size_t work_bytes = std::max(tmp1, tmp2), at_work = place(work_bytes), at_S = place(4 * nown * t.sstride),
                at_row = place(4 * nown), at_pa = place(4 * nown), at_pb = place(4 * nown), at_ra = place(4 * nown),
-               at_rb = place(4 * nown), at_k = place(8 * nown), at_ks = place(8 * nown);
+               at_rb = place(4 * nown), at_k = place(8 * nown), at_ks = place(8 * nown), at_g = place(8);
   PoolBuf tmp(used, st, size_t(256) << 20);
   char *const base = tmp.as<char>();
   const U32 S_piv = U32(base + at_S), own_row = U32(base + at_row), perm_a = U32(base + at_pa),
@@ -1085,8 +1088,11 @@ ChainData &chain_data(TensorState &t) {
     chain_gather_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_a, nown, t.sstride, S_piv, t.own_c64.p, cd->S.p,
                                                                cd->c64.p, cd->c32.p);
     SPB_LAUNCH_CHECK();
-    chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S.p, rows_b, nown, t.sstride, L, cd->flags.p);
+    unsigned long long *const groups = reinterpret_cast<unsigned long long *>(base + at_g);
+    SPB_CUDA(cudaMemsetAsync(groups, 0, sizeof(*groups), st));
+    chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S.p, rows_b, nown, t.sstride, L, cd->flags.p, groups);
     SPB_LAUNCH_CHECK();
+    SPB_CUDA(cudaMemcpyAsync(&cd->ngroups, groups, sizeof(*groups), cudaMemcpyDeviceToHost, st));
   }
   SPB_CUDA(cudaDeviceSynchronize());
   t.chain = cd;
@@ -1104,7 +1110,7 @@ ChainData &chain_data(TensorState &t) {
 ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturing) {
   ChainData &cd = chain_data(t);
   const bool warp = chain8_supported(t, R);
-  const bool groups = !cd.no_groups && chain5_pays(t, R, precision);
+  const bool groups = !cd.no_groups && chain5_pays(t, cd, R, precision);
   std::unique_ptr<ChainItems> &slot = cd.items[warp || groups], &other = cd.items[!(warp || groups)];
   if (slot) return *slot;
   if (other && (capturing || (t.order == 5 && !groups))) return *other;
@@ -1291,7 +1297,7 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
     // the tables of both kernels of a rank, so that either can be captured once one has run
     order5_tables(R);
     chain5_tables(R);
-    if (items.groups && chain5_pays(t, R, precision)) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
+    if (items.groups && chain5_pays(t, cd, R, precision)) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
     else chain5_rows_launch(t, cd, items, dU, R, dYpacked, precision, st);
     return;
   }

@@ -36,6 +36,7 @@ struct ChainData {
   DBuf<double> c64;               // owner coefficients in chain order
   DBuf<float> c32;
   DBuf<uint8_t> flags;            // bit k: the owner starts a new prefix of k+1 pivots
+  uint64_t ngroups = 0;           // runs of owners of a row with the same first pivot
   std::unique_ptr<ChainGroups> groups;
   bool no_groups = false;         // no memory for them: the CTA kernel runs instead
   // items, by kernel: the CTA kernels; the warp kernel (order 4, R <= 8) or the
@@ -68,7 +69,7 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
 // the owners of items (ranges in row order of the owners in pivot order), dealt to
 // its warps; one pass over items whose ob is the item's number in row order and
 // whose oe - ob is its number of sub-groups.
-bool chain5_pays(const TensorState &t, uint32_t R, int precision);
+bool chain5_pays(const TensorState &t, const ChainData &cd, uint32_t R, int precision);
 void chain5_tables(uint32_t R);  // its index table of a rank, built on first use
 std::unique_ptr<ChainGroups> chain5_build(const TensorState &t, const ChainData &cd, const std::vector<Chunk> &items);
 void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &items, const void *dU, uint32_t R,

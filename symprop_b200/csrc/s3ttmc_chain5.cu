@@ -48,7 +48,18 @@
 // 104 a thread of 128); FP32 at R > 8 comes here where a node has 64 owners on
 // average, because closing an item (all of G through shared memory) costs as much
 // as some tens of owners (at 25 owners a node the two are equal, at 10 this one
-// takes 1.15 times as long, at 200 it is the faster one).
+// takes 1.15 times as long, at 200 it is the faster one), and at R > 12 only with at
+// least one group (s_1) to 10 owners: the CTA kernel gains from owners that share
+// pivots, this one hardly.  FP32, R = 16, ms, CTA kernel / this one, by groups an owner:
+//   1,000 nodes, 200,000 equal degrees    0.43    1.778  0.980
+//   20,000, 2,000,000 power-law           0.19    6.82   5.41
+//   20,000, 300,000 Zipf(1.05)            0.155   1.693  1.446
+//   3,000, 60,000 Zipf(1.1)               0.103   0.272  0.271
+//   10,000, 400,000 Zipf(1.1)             0.078   1.344  1.346
+//   1,000, 20,000 Zipf(1.2)               0.069   0.095  0.104
+//   1,000, 50,000 Zipf(1.2)               0.043   0.156  0.177
+//   3,000, 600,000 Zipf(1.1)              0.035   1.307  1.460
+// (R = 12 on the last one: 1.331 / 0.980.)
 //
 // The first call on a tensor also orders its owners (chain_data: two radix sorts)
 // and deals them to the warps (chain5_build); both are kept.  First call, ms, FP32,
@@ -597,10 +608,11 @@ template <typename T> void dispatch(const GroupParams &p, cudaStream_t st) {
 void chain5_tables(uint32_t R) { quad_table(R); }
 
 // both sides of each line: the table above
-bool chain5_pays(const TensorState &t, uint32_t R, int precision) {
+bool chain5_pays(const TensorState &t, const ChainData &cd, uint32_t R, int precision) {
   if (t.order != 5 || !chain_supported(t, R) || t.sstride != 4) return false;
   if (precision == SYMPROP_FP64) return R <= 12;
-  return R <= 8 || t.nown >= 64ull * t.dim;
+  if (R <= 8) return true;
+  return t.nown >= 64ull * t.dim && (R <= 12 || 10 * cd.ngroups >= t.nown);
 }
 
 std::unique_ptr<ChainGroups> chain5_build(const TensorState &t, const ChainData &cd, const std::vector<Chunk> &items) {
