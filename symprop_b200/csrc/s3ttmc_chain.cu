@@ -1113,7 +1113,7 @@ ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturin
   const bool groups = !cd.no_groups && chain5_pays(t, cd, R, precision);
   std::unique_ptr<ChainItems> &slot = cd.items[warp || groups], &other = cd.items[!(warp || groups)];
   if (slot) return *slot;
-  if (other && (capturing || (t.order == 5 && !groups))) return *other;
+  if (other && capturing) return *other;
   auto it = std::make_unique<ChainItems>();
   const uint64_t target_items = 148ull * 32ull;
   const uint64_t co = (heavy_owner_count(t) + target_items - 1) / target_items;
