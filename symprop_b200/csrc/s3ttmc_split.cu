@@ -37,6 +37,8 @@
 // (mod 16) doubles apart: the fragments' 8-byte loads are free of bank
 // conflicts.
 #include <algorithm>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "check.cuh"
@@ -377,8 +379,17 @@ bool split_supported(uint32_t order, uint32_t R) { return order == kL + 1 && R >
 // is the slower one at every length.
 uint32_t split_heavy(uint32_t R, const ItemSet &items) { return R <= 8 ? items.nheavy : items.nchunks; }
 
+// The tables of a rank are kept per device for the life of the process (at most 43 KB
+// each): made for every tensor they were a third of the first call on a small one (order 6,
+// 4,000 tuples, R = 4, FP32).
 std::shared_ptr<SplitPlan> split_plan(uint32_t order, uint32_t R) {
   if (!split_supported(order, R)) fail(SYMPROP_ERR_SIZE, "split S3TTMc does not support order %u rank %u", order, R);
+  static std::mutex mu;
+  static auto &plans = *new std::map<std::pair<int, uint32_t>, std::shared_ptr<SplitPlan>>;  // outlives the context
+  int dev = 0;
+  SPB_CUDA(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lk(mu);
+  if (const auto it = plans.find({dev, R}); it != plans.end()) return it->second;
   auto pl = std::make_shared<SplitPlan>();
   pl->R = R;
   pl->m = (uint32_t)symsize(R, kL);
@@ -418,7 +429,7 @@ std::shared_ptr<SplitPlan> split_plan(uint32_t order, uint32_t R) {
   SPB_CUDA(cudaMemcpy(pl->pairs.p, pairs.data(), pairs.size() * 4, cudaMemcpyHostToDevice));
   pl->sym.alloc(sym.size());
   SPB_CUDA(cudaMemcpy(pl->sym.p, sym.data(), sym.size() * 4, cudaMemcpyHostToDevice));
-  return pl;
+  return plans[{dev, R}] = pl;
 }
 
 void split_launch(const SplitPlan &pl, const TensorState &t, const ItemSet &items, const void *dU, void *dYpacked,
