@@ -37,7 +37,7 @@
 // Bound: 16 int8 products over the upper 256 x 256 tiles.  200,000 x 3,876:
 // 136 tiles, 5.7e13 integer operations (12.7 ms at the nominal 4.5 POP/s),
 // against 3.0e12 FP64 operations (81 ms at the nominal 37 TFLOP/s) for the
-// CUDA-core kernel in dense.cu (137 ms).  Measured 27.6 ms: product 17.9 (3.2
+// CUDA-core kernel in dense.cu (137 ms).  Measured 27.4 ms (with the check 28.4): product 17.9 (3.2
 // POP/s), residues 5.8 (reads A, writes 16 bytes per entry), remainders 1.1,
 // column maxima 0.9; error against 64 bits 1.2e-16, 6.2e-15 for the CUDA-core
 // kernel.  Running the residues and remainders on a second stream beside the
@@ -245,15 +245,19 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 
 struct I8Args {
   int cols, ntile, ntiles;    // tiles of 256 per side, upper tiles
-  int kblocks;                // 128-wide blocks of a chunk
+  int kblocks, kstep;         // 128-wide blocks of a chunk: how many, every kstep-th
   unsigned char *C;           // (chunk * kP + p) planes of ld x ld residues
   int ld;
   int *err;
   uint64_t wait_ns;
   int expired_warp;           // failure injection (-1: none)
   int planes;                 // per chunk: kP of residues, one more of magnitudes
-  int nchunk;                 // of this launch
-  // magnitudes: entries to be summed in FP64 go to the list
+  // The first `checks` units are the products of the chunks' magnitudes: over some of the
+  // rows (some: *suspect is set when an entry may have to be summed in FP64) or
+  // over all (such entries go to the list; with `suspect` only when that is set).
+  int checks;
+  bool some;
+  int *suspect;
   const unsigned long long *nsq;
   int chunk0, chunk, rows;
   Odd odd;
@@ -269,11 +273,13 @@ __global__ void __launch_bounds__(256, 1)
   __shared__ volatile int progress;
   __shared__ int issued[kNStages];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // unit: tile fastest, so that the CTAs of a wave share a modulus in L2; the
-  // magnitudes of all chunks first
-  const int unit = (int)blockIdx.x / a.ntiles, checks = (a.planes - kP) * a.nchunk, residues = unit - checks;
-  const int plane = residues < 0 ? unit * a.planes + kP : residues / kP * a.planes + residues % kP;
-  if (checks && __syncthreads_or(threadIdx.x == 0 && a.odd.too_many())) return;
+  // unit: tile fastest, so that the CTAs of a wave share a modulus in L2
+  const int unit = (int)blockIdx.x / a.ntiles, sums = unit - a.checks;
+  const bool check = sums < 0;
+  const int plane = check ? unit * a.planes + kP : sums / kP * a.planes + sums % kP;
+  if (a.planes > kP &&
+      __syncthreads_or(threadIdx.x == 0 && (a.odd.too_many() || (check && !a.some && a.suspect && !*a.suspect))))
+    return;
   int ti = 0, tj = (int)blockIdx.x - unit * a.ntiles;
   while (tj >= a.ntile - ti) {
     tj -= a.ntile - ti;
@@ -294,7 +300,6 @@ __global__ void __launch_bounds__(256, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const int chunk = a.chunk0 + plane / a.planes, modulus = plane % a.planes;
-  const bool check = modulus == kP;
   __shared__ float norm[kTile];  // check: N of the tile's columns, 0 past the last
   const unsigned long long *nsq = a.nsq + (size_t)chunk * a.cols;
   if (check) {
@@ -322,8 +327,8 @@ __global__ void __launch_bounds__(256, 1)
       }
       unsigned char *st = smem + (size_t)s * 2 * kOperand;
       mbar_expect_tx(&full_bar[s], 2 * kOperand);
-      tma_load_2d(st, &map, &full_bar[s], it * kBK, row0);
-      tma_load_2d(st + kOperand, &map, &full_bar[s], it * kBK, col0);
+      tma_load_2d(st, &map, &full_bar[s], it * a.kstep * kBK, row0);
+      tma_load_2d(st + kOperand, &map, &full_bar[s], it * a.kstep * kBK, col0);
       issued[s] = it + 1;
     }
   } else if (warp == 1 && lane == 0) {
@@ -367,6 +372,10 @@ __global__ void __launch_bounds__(256, 1)
         const float nj = norm[c + q];
         const int j = tj * kTile + c + q;
         if (ni > 0.f && nj > 0.f && i <= j && !(ni + nj <= unit * (float)(int)v[q])) {
+          if (a.some) {
+            *a.suspect = 1;
+            continue;
+          }
           // past the limit the count no longer matters (and may not wrap)
           if (a.odd.too_many()) continue;
           const unsigned at = atomicAdd(a.odd.count, 1u);
@@ -500,10 +509,16 @@ int sms() {
 // (latency) and 75 us at 2,002: of the chunk counts whose operands, chunk by chunk, take at
 // most `limit` bytes, the one whose waves take least.  `nchunk` is 0 when there is
 // none.
+// The check of a componentwise Gram is a 17th plane among the sums, or (some rows give
+// a lower bound of W as well) two launches before them: every kstep-th block of 128 rows,
+// and all rows only where that is not enough.  The second costs two launches, the
+// first often a wave: 200,000 x 3,876 29.9 / 28.6 ms (without a check 27.4), 20,000 x
+// 2,002 1.15 / 1.09 (1.03); 20,000 x 320 0.315 / 0.333, 1,536 x 715 0.150 / 0.182.
 struct I8Plan {
   int ntile, ntiles, ld;
   int chunk, nchunk = 0;    // rows per chunk
   int kc, group;            // padded rows, chunks per launch
+  int kstep = 1;            // above 1: the check by itself, over every kstep-th block of rows first
   size_t res, bytes;        // of a launch's residues, and of all its operands
 };
 
@@ -529,16 +544,27 @@ I8Plan plan_i8(int rows, int cols, int planes, size_t limit) {
     const int kc = ((rows + c - 1) / c + kBK - 1) / kBK * kBK;
     int group = c;
     while (group > 1 && bytes(kc, group) > limit) --group;
-    double t = c * std::max(35000.0, 0.035 * cols * cols);
-    for (int x = 0; x < c; x += group) {
-      const double units = (double)g.ntiles * planes * std::min(group, c - x);
-      t += std::ceil(units / n) * (kc / kBK * 1024.0 + 12000.0);
-    }
-    if (t < best) {
-      best = t;
-      g.nchunk = (rows + kc - 1) / kc;
-      g.kc = kc;
-      g.group = group;
+    // with the check among the sums' units, or (kstep > 1) before them
+    auto clocks = [&](int kstep) {
+      double t = c * std::max(35000.0, 0.035 * cols * cols);
+      auto launch = [&](double units, int kblocks) { t += std::ceil(units / n) * (kblocks * 1024.0 + 12000.0); };
+      for (int x = 0; x < c; x += group) {
+        const double part = (double)g.ntiles * std::min(group, c - x);
+        launch(part * (kstep > 1 ? kP : planes), kc / kBK);
+        if (kstep > 1) launch(part, kc / kBK / kstep), t += 50000.0;
+      }
+      return t;
+    };
+    const int some = planes > kP ? std::max(1, std::min(8, kc / kBK / 8)) : 1;
+    for (int kstep : {1, some}) {
+      const double t = clocks(kstep);
+      if (t < best) {
+        best = t;
+        g.nchunk = (rows + kc - 1) / kc;
+        g.kc = kc;
+        g.group = group;
+        g.kstep = kstep;
+      }
     }
   }
   g.chunk = (rows + g.nchunk - 1) / g.nchunk;  // chunks of like length: no short last one
@@ -551,20 +577,20 @@ I8Plan plan_i8(int rows, int cols, int planes, size_t limit) {
 
 }  // namespace
 
-// Six launches, two waits and 256-wide tiles take 130 us and more, so that the FP64
-// kernels win where they are not at their own worst: us, FP64 kernel / this one:
-//   rows                     1,536      3,000      6,000      10,000     40,000
-//   320 columns (even)     336 / 146  329 / 155  270 / 178  286 / 246  1,025 / 413
-//   321 (odd, gemm)         66 / 144   96 / 153  173 / 168  254 / 244    983 / 403
-//   513                    109 / 153  180 / 161  324 / 234  516 / 281  2,057 / 552
-//   816                    338 / 172  335 / 230  280 / 304  439 / 367  1,628 / 803
-//   2,002                  365 / 376  662 / 448  1,261 / 566  2,059 / 716  8,048 / 2,018
+// Six launches, two waits and 256-wide tiles take 110 us and more, so that gemm's
+// FP64 tiles win at odd widths of few rows (gram_f64, even widths, does not).  us, FP64
+// kernel / this one with the check:
+//   rows                     1,536      3,000      6,000      10,000     80,000
+//   320 columns (even)     332 / 115  326 / 129  266 / 156  281 / 197  2,011 / 567
+//   321 (odd)               66 / 119   96 / 132  175 / 146  257 / 181  1,934 / 557
+//   513                    108 / 127  181 / 142  324 / 179  515 / 210  4,103 / 863
+//   816                    337 / 157  333 / 182  277 / 235  438 / 304  3,209 / 1,363
+//   2,002                  364 / 317  662 / 381  1,261 / 506  2,059 / 653  16,025 / 3,686
 // The caller compares the two times (f64_gram_us in dense.cu).  This one is fitted to
-// where they meet, over 190 sizes of 1,536 to 80,000 rows and 320 to 2,002 columns: the
-// slower kernel is taken at five of them, and then by at most 10%.  Not below 320
-// columns or 1,536 rows, where it was not measured to win.
+// where they meet: over 190 sizes of 1,536 to 80,000 rows and 320 to 2,002 columns the
+// faster kernel is taken at every one.  Below, only the FP64 kernels.
 bool i8_gram_takes(int rows, int cols) { return cols >= 320 && rows >= 1536; }
-double i8_gram_us(int rows, int cols) { return 80.0 + 0.01 * rows + 0.04 * cols + 1e-5 * rows * cols; }
+double i8_gram_us(int rows, int cols) { return 70.0 + 0.002 * rows + 0.06 * cols + 1.5e-5 * rows * cols; }
 
 // Entries that the caller of a componentwise Gram may have summed one by one: 64
 // bytes of A a row each, against cols^2 / 2 FMAs a row for all of them by the FP64
@@ -594,11 +620,14 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
   signed char *const res = ops->as<signed char>();
   unsigned char *const rem = ops->as<unsigned char>() + g.res;
   const size_t ncs = (size_t)g.nchunk * cols;
-  PoolBuf cmax(ncs * 8, st), sc(ncs * 4, st), flags(3 * sizeof(int), st);
+  PoolBuf cmax(ncs * 8, st), sc(ncs * 4, st), flags(4 * sizeof(int), st);
   int *bad = (int *)flags.p, *err = bad + 1;
   SPB_CUDA(cudaMemsetAsync(cmax.p, 0, ncs * 8, st));
-  SPB_CUDA(cudaMemsetAsync(flags.p, 0, 3 * sizeof(int), st));
-  const int part = 512;
+  SPB_CUDA(cudaMemsetAsync(flags.p, 0, 4 * sizeof(int), st));
+  // a CTA walks its rows in 0.15 us each, so 8 CTAs an SM where there are rows for them
+  // (512 rows a CTA: 80 us from 1,536 x 320 to 80,000 x 320)
+  const int ctas = (cols + 127) / 128 * g.nchunk, parts = (8 * sms() + ctas - 1) / ctas,
+            part = std::min(512, std::max(32, (g.chunk + parts - 1) / parts));
   col_max_kernel<<<dim3((cols + 127) / 128, g.nchunk, (g.chunk + part - 1) / part), 128, 0, st>>>(
       A, rows, cols, lda, g.chunk, part, (unsigned long long *)cmax.p);
   SPB_LAUNCH_CHECK();
@@ -613,11 +642,9 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     return !h[0] && (unsigned)h[2] <= max_pairs(cols);
   };
   if (!read_flags()) return false;
-  // The check of a componentwise Gram runs with the residues and their product.  By
-  // itself before them it would cost more where it passes (200,000 x 3,876: 29.8 instead
-  // of 28.2 ms; 10,000 x 816: 0.443 instead of 0.409 ms; without a check 27.2 and 0.405).
   PoolBuf list(componentwise ? max_pairs(cols) * sizeof(int2) : 0, st), nsq(componentwise ? ncs * 8 : 0, st);
   const Odd odd{list.as<int2>(), (unsigned *)(bad + 2), max_pairs(cols)};
+  int *const suspect = bad + 3;
   if (componentwise) SPB_CUDA(cudaMemsetAsync(nsq.p, 0, ncs * 8, st));
   SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   for (int c0 = 0; c0 < g.nchunk; c0 += g.group) {
@@ -639,21 +666,33 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     a.cols = cols;
     a.ntile = g.ntile;
     a.ntiles = g.ntiles;
-    a.kblocks = g.kc / kBK;
     a.C = rem;
     a.ld = g.ld;
     a.err = err;
     a.wait_ns = mainloop_wait_ns();
     a.expired_warp = expired_warp();
     a.planes = planes;
-    a.nchunk = nc;
     a.nsq = (const unsigned long long *)nsq.p;
     a.chunk0 = c0;
     a.chunk = g.chunk;
     a.rows = rows;
     a.odd = odd;
-    i8_gram_kernel<<<(unsigned)(g.ntiles * planes * nc), 256, kSmem, st>>>(map, a);
-    SPB_LAUNCH_CHECK();
+    auto product = [&](int checks, bool sums, int kstep = 1, bool some = false, int *suspect = nullptr) {
+      a.checks = checks;
+      a.some = some;
+      a.suspect = suspect;
+      a.kstep = kstep;
+      a.kblocks = (g.kc / kBK + kstep - 1) / kstep;
+      i8_gram_kernel<<<(unsigned)(g.ntiles * (checks + (sums ? nc * kP : 0))), 256, kSmem, st>>>(map, a);
+      SPB_LAUNCH_CHECK();
+    };
+    if (g.kstep > 1) {
+      product(nc, false, g.kstep, true, suspect);
+      product(nc, false, 1, false, suspect);
+      product(0, true);
+    } else {
+      product(componentwise ? nc : 0, true);
+    }
     const unsigned nt = (unsigned)((cols + 31) / 32);
     crt_kernel<<<dim3(nt, nt), 256, 0, st>>>(rem, g.ld, cols, nc, c0, (const int *)sc.p,
                                              c0 > 0 ? 1 : 0, C, ldc, odd);
