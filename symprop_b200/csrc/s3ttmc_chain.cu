@@ -476,8 +476,6 @@ template <bool MMA> constexpr int kFStride = kRP * kS2 + (MMA ? 4 : 0);
 
 struct Chain5Params {
   const Chunk *chunks;
-  const uint32_t *first;  // items of the group kernel (ChainGroups), null: ranges of owners
-  uint64_t nitems;
   uint32_t nchunks;
   const uint32_t *S;  // nown x 4 leaf ids in pivot order
   const void *c;
@@ -523,13 +521,7 @@ __global__ void __launch_bounds__(kThreads5, (sizeof(T) == 8 ? 1 : 2)) s3ttmc_ch
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem5<T, MMA> &sm = *reinterpret_cast<Smem5<T, MMA> *>(smem_raw);
   const int tid = threadIdx.x;
-  Chunk ch = p.chunks[blockIdx.x];
-  if (p.first) {  // an item of the group kernel: its number in ob
-    if (!SPB_BOUND(ch.ob < p.nitems, 211, blockIdx.x)) return;
-    const uint32_t *f = p.first + ch.ob * kGroupPlaces;
-    ch.ob = f[0];
-    ch.oe = f[kGroupPlaces - 1];
-  }
+  const Chunk ch = p.chunks[blockIdx.x];
   if (!SPB_BOUND(ch.ob <= ch.oe && ch.oe <= p.nown && ch.row < p.nrows && (ch.slot == kDirect || ch.slot < p.nslots),
                  211, blockIdx.x))
     return;
@@ -1114,14 +1106,12 @@ ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturin
   std::unique_ptr<ChainItems> &slot = cd.items[warp || groups], &other = cd.items[!(warp || groups)];
   if (slot) return *slot;
   if (other && capturing) return *other;
-  auto it = std::make_unique<ChainItems>();
   const uint64_t target_items = 148ull * 32ull;
-  const uint64_t co = (heavy_owner_count(t) + target_items - 1) / target_items;
-  it->chunk_owners = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(co, warp ? 64 : 256), 1024);
-  it->groups = groups;
+  const uint64_t most = (heavy_owner_count(t) + target_items - 1) / target_items;
+  const uint32_t co = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(most, warp ? 64 : 256), 1024);
   std::vector<Chunk> ch, lt;
   std::vector<SplitRow> sp;
-  it->nslots = cut_chain_rows(t, it->chunk_owners, 0, t.dim, ch, sp, lt);
+  const uint32_t nslots = cut_chain_rows(t, co, 0, t.dim, ch, sp, lt);
   if (groups && !cd.groups) {
     try {
       cd.groups = chain5_build(t, cd, ch);
@@ -1131,15 +1121,23 @@ ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturin
       return chain_items(t, R, precision, capturing);
     }
   }
-  sort_chain_items(cd, *it, ch, 0, ch.size());
   sort_heaviest_first(lt, 0, lt.size(), kChainLight);
-  it->nchunks = (uint32_t)ch.size();
-  it->nsplit = (uint32_t)sp.size();
-  it->nlight = (uint32_t)lt.size();
-  upload(it->chunks, ch);
-  upload(it->split, sp);
-  upload(it->light, lt);
-  return *(slot = std::move(it));
+  auto make = [&](bool of_groups, std::vector<Chunk> list) {
+    auto it = std::make_unique<ChainItems>();
+    it->chunk_owners = co;
+    it->groups = of_groups;
+    it->nslots = nslots;
+    sort_chain_items(cd, *it, list, 0, list.size());
+    it->nchunks = (uint32_t)list.size();
+    it->nsplit = (uint32_t)sp.size();
+    it->nlight = (uint32_t)lt.size();
+    upload(it->chunks, list);
+    upload(it->split, sp);
+    upload(it->light, lt);
+    return it;
+  };
+  if (groups && !other) other = make(false, ch);  // for calls that are captured
+  return *(slot = make(groups, std::move(ch)));
 }
 
 const ChainItems *built_chain_items(const TensorState &t, uint32_t R) {
@@ -1255,8 +1253,6 @@ void chain5_rows_launch(const TensorState &t, const ChainData &cd, const ItemSet
   const Order5Tables &tb = order5_tables(R);
   Chain5Params p;
   p.chunks = items.chunks;
-  p.first = items.groups ? cd.groups->first.p : nullptr;
-  p.nitems = items.groups ? cd.groups->sub.size() : 0;
   p.nchunks = items.nchunks;
   p.S = cd.S.p;
   p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64.p : (const void *)cd.c32.p;
@@ -1297,7 +1293,7 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
     // the tables of both kernels of a rank, so that either can be captured once one has run
     order5_tables(R);
     chain5_tables(R);
-    if (items.groups && chain5_pays(t, cd, R, precision)) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
+    if (items.groups) chain5_launch(t, cd, items, dU, R, dYpacked, precision, st);
     else chain5_rows_launch(t, cd, items, dU, R, dYpacked, precision, st);
     return;
   }

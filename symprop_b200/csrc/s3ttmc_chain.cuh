@@ -21,7 +21,6 @@ struct ChainItems {
 
 // Order 5: the owners of every item in the order the building warps of
 // s3ttmc_chain5.cu take them.  Built on first use of a rank it covers.
-constexpr int kGroupPlaces = 9;  // of an item in `first`
 struct ChainGroups {
   DBuf<uint32_t> S;               // nown x 4 leaf ids in pivot order; bit 31 of s_1: ends its sub-group
   DBuf<double> c;                 // owner coefficients
@@ -55,9 +54,9 @@ bool chain_supported(const TensorState &t, uint32_t R);
 // The chain data of t (built on the first call).
 ChainData &chain_data(TensorState &t);
 // The work items of a rank and precision (built on first use), and in nb row bands.
-// Either list of an order serves all its kernels: while a stream is captured, when
-// none can be built, the one that is there does.  (Otherwise each has its own: the CTA
-// kernel of order 5 loses up to 4% with the group kernel's order of items.)
+// While a stream is captured, when none can be built, another kernel's list does: at
+// order 4 either serves both kernels, at order 5 the CTA kernel's is made together with
+// the group kernel's.
 ChainItems &chain_items(TensorState &t, uint32_t R, int precision, bool capturing = false);
 const ChainItems *built_chain_items(const TensorState &t, uint32_t R);  // null before the first use
 const RowBands &chain_bands(TensorState &t, ChainItems &items, uint32_t nb);

@@ -85,8 +85,7 @@ constexpr int kSub = 16;         // owners per sub-group
 template <typename T> constexpr int kBlk = sizeof(T) == 8 ? 2 : 4;  // owners gathered at a time by a warp
 constexpr int kStages = 2;
 constexpr uint32_t kLast = 0x80000000u;
-constexpr int kFirst = kGroupPlaces;
-static_assert(kFirst == kBuildWarps + 1, "places of an item in `first`");
+constexpr int kFirst = kBuildWarps + 1;  // places of an item in `first`
 
 // Places of T: by the middle index y, then z, then x (the lanes of a set, pairs
 // with the same y next to each other, store next to each other).
