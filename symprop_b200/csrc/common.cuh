@@ -163,6 +163,44 @@ struct PoolBuf {
   template <class T> T *as() const { return reinterpret_cast<T *>(p); }
 };
 
+// What a tensor keeps after its first call, several arrays in one allocation: of the pool
+// up to kPoolMax, where it takes a few us (cudaMalloc takes 0.4 ms from 1 MB on).  Freed
+// when the device is done with it, on whichever stream.
+struct KeptBuf {
+  static constexpr size_t kPoolMax = size_t(64) << 20;
+  char *p = nullptr;
+  int dev = 0;
+  bool pooled = false;
+  KeptBuf() = default;
+  KeptBuf(const KeptBuf &) = delete;
+  KeptBuf &operator=(const KeptBuf &) = delete;
+  void alloc(size_t bytes, cudaStream_t st) {
+    if (!bytes) return;
+    SPB_CUDA(cudaGetDevice(&dev));
+    pooled = bytes <= kPoolMax;
+    p = static_cast<char *>(device_alloc(bytes, pooled ? device_pool() : nullptr, st));
+  }
+  ~KeptBuf() {
+    if (!p) return;
+    int cur = dev;
+    cudaGetDevice(&cur);
+    if (cur != dev) cudaSetDevice(dev);
+    if (pooled) cudaDeviceSynchronize();  // cudaFree does not wait for memory of a pool
+    cudaFree(p);
+    if (cur != dev) cudaSetDevice(cur);
+  }
+};
+
+// Places of arrays that share one allocation, each on 256 bytes.
+struct Places {
+  size_t bytes = 0;
+  template <class T> size_t add(size_t count) {
+    const size_t at = bytes;
+    bytes += (count * sizeof(T) + 255) / 256 * 256;
+    return at;
+  }
+};
+
 // ------------------------------------------------------- packed indexing
 
 inline uint64_t binom(uint64_t n, uint64_t k) {

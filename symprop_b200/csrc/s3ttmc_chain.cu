@@ -1038,26 +1038,32 @@ ChainData &chain_data(TensorState &t) {
   const int bits = bits_for(n ? n - 1 : 0);
   const int key_bits = bits * (int)(L - 1);
   if (key_bits > 64) fail(SYMPROP_ERR_SIZE, "chain schedule: pivot key of %d bits", key_bits);
-  // Temporaries in one buffer, of the pool up to 256 MB: nine allocations and frees of
-  // their own took two thirds of a first call (6 of 8.3 ms at 1M owners).
-  size_t tmp1 = 0, tmp2 = 0, used = 0;
+  // Temporaries in one buffer, of the pool up to 256 MB, and what is kept in another:
+  // thirteen allocations of their own took most of a first call (7 of 8.3 ms at 1M
+  // owners).
   using U32 = uint32_t *;
   using U64 = uint64_t *;
+  size_t tmp1 = 0, tmp2 = 0;
   SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp1, U64(), U64(), U32(), U32(), nown, 0, std::max(key_bits, 1), st));
   SPB_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp2, U32(), U32(), U32(), U32(), nown, 0, bits_for(n), st));
-  auto place = [&](size_t bytes) {
-    const size_t at = used;
-    used += (bytes + 255) / 256 * 256;
-    return at;
-  };
-  const size_t work_bytes = std::max(tmp1, tmp2), at_work = place(work_bytes), at_S = place(4 * nown * t.sstride),
-               at_row = place(4 * nown), at_pa = place(4 * nown), at_pb = place(4 * nown), at_ra = place(4 * nown),
-               at_rb = place(4 * nown), at_k = place(8 * nown), at_ks = place(8 * nown), at_g = place(8);
-  PoolBuf tmp(used, st, size_t(256) << 20);
+  const size_t work_bytes = std::max(tmp1, tmp2);
+  Places pl, kept;
+  const size_t at_work = pl.add<char>(work_bytes), at_S = pl.add<uint32_t>(nown * t.sstride),
+               at_row = pl.add<uint32_t>(nown), at_pa = pl.add<uint32_t>(nown), at_pb = pl.add<uint32_t>(nown),
+               at_ra = pl.add<uint32_t>(nown), at_rb = pl.add<uint32_t>(nown), at_k = pl.add<uint64_t>(nown),
+               at_ks = pl.add<uint64_t>(nown), at_g = pl.add<unsigned long long>(1);
+  PoolBuf tmp(pl.bytes, st, size_t(256) << 20);
   char *const base = tmp.as<char>();
   const U32 S_piv = U32(base + at_S), own_row = U32(base + at_row), perm_a = U32(base + at_pa),
             perm_b = U32(base + at_pb), rows_a = U32(base + at_ra), rows_b = U32(base + at_rb);
   const U64 pkey = U64(base + at_k), pkey_sorted = U64(base + at_ks);
+  const size_t kept_S = kept.add<uint32_t>(nown * t.sstride), kept_c64 = kept.add<double>(nown),
+               kept_c32 = kept.add<float>(nown), kept_f = kept.add<uint8_t>(nown);
+  cd->store.alloc(kept.bytes, st);
+  cd->S = U32(cd->store.p + kept_S);
+  cd->c64 = reinterpret_cast<double *>(cd->store.p + kept_c64);
+  cd->c32 = reinterpret_cast<float *>(cd->store.p + kept_c32);
+  cd->flags = reinterpret_cast<uint8_t *>(cd->store.p + kept_f);
   if (nown) {
     pivot_order_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(t.own_S.p, nown, t.sstride, L, rank, bits, S_piv, pkey);
     SPB_LAUNCH_CHECK();
@@ -1071,18 +1077,12 @@ ChainData &chain_data(TensorState &t) {
     SPB_LAUNCH_CHECK();
     SPB_CUDA(cub::DeviceRadixSort::SortPairs(base + at_work, bytes, rows_a, rows_b, perm_b, perm_a, nown, 0,
                                              bits_for(n), st));
-  }
-  cd->S.alloc(nown * t.sstride);
-  cd->c64.alloc(nown);
-  cd->c32.alloc(nown);
-  cd->flags.alloc(nown);
-  if (nown) {
-    chain_gather_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_a, nown, t.sstride, S_piv, t.own_c64.p, cd->S.p,
-                                                               cd->c64.p, cd->c32.p);
+    chain_gather_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(perm_a, nown, t.sstride, S_piv, t.own_c64.p, cd->S,
+                                                               cd->c64, cd->c32);
     SPB_LAUNCH_CHECK();
     unsigned long long *const groups = reinterpret_cast<unsigned long long *>(base + at_g);
     SPB_CUDA(cudaMemsetAsync(groups, 0, sizeof(*groups), st));
-    chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S.p, rows_b, nown, t.sstride, L, cd->flags.p, groups);
+    chain_flags_kernel<<<blocks_for(nown, 256), 256, 0, st>>>(cd->S, rows_b, nown, t.sstride, L, cd->flags, groups);
     SPB_LAUNCH_CHECK();
     SPB_CUDA(cudaMemcpyAsync(&cd->ngroups, groups, sizeof(*groups), cudaMemcpyDeviceToHost, st));
   }
@@ -1254,9 +1254,9 @@ void chain5_rows_launch(const TensorState &t, const ChainData &cd, const ItemSet
   Chain5Params p;
   p.chunks = items.chunks;
   p.nchunks = items.nchunks;
-  p.S = cd.S.p;
-  p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64.p : (const void *)cd.c32.p;
-  p.flags = cd.flags.p;
+  p.S = cd.S;
+  p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64 : (const void *)cd.c32;
+  p.flags = cd.flags;
   p.U = dU;
   p.R = R;
   p.m2 = R * (R + 1) / 2;
@@ -1304,10 +1304,10 @@ void chain_launch(const TensorState &t, const ChainData &cd, const ItemSet &item
   ChainParams p;
   p.chunks = items.chunks;
   p.nchunks = items.nchunks;
-  p.S = cd.S.p;
+  p.S = cd.S;
   p.sstride = t.sstride;
-  p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64.p : (const void *)cd.c32.p;
-  p.flags = cd.flags.p;
+  p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64 : (const void *)cd.c32;
+  p.flags = cd.flags;
   p.U = dU;
   p.R = R;
   p.m2 = R * (R + 1) / 2;

@@ -22,19 +22,21 @@ struct ChainItems {
 // Order 5: the owners of every item in the order the building warps of
 // s3ttmc_chain5.cu take them.  Built on first use of a rank it covers.
 struct ChainGroups {
-  DBuf<uint32_t> S;               // nown x 4 leaf ids in pivot order; bit 31 of s_1: ends its sub-group
-  DBuf<double> c;                 // owner coefficients
-  DBuf<uint32_t> first;           // per item in row order: the first owner of each warp, the item's end
+  KeptBuf store;                  // of the arrays
+  uint32_t *S = nullptr;          // nown x 4 leaf ids in pivot order; bit 31 of s_1: ends its sub-group
+  double *c = nullptr;            // owner coefficients
+  uint32_t *first = nullptr;      // per item in row order: the first owner of each warp, the item's end
   std::vector<uint32_t> sub;      // per item: its sub-groups
 };
 
 // Owners re-sorted for the chain schedule, built on first use.
 struct ChainData {
   uint32_t L = 0;                 // leaf size (order - 1)
-  DBuf<uint32_t> S;               // nown x sstride leaf ids, highest-degree first
-  DBuf<double> c64;               // owner coefficients in chain order
-  DBuf<float> c32;
-  DBuf<uint8_t> flags;            // bit k: the owner starts a new prefix of k+1 pivots
+  KeptBuf store;                  // of the arrays
+  uint32_t *S = nullptr;          // nown x sstride leaf ids, highest-degree first
+  double *c64 = nullptr;          // owner coefficients in chain order
+  float *c32 = nullptr;
+  uint8_t *flags = nullptr;       // bit k: the owner starts a new prefix of k+1 pivots
   uint64_t ngroups = 0;           // runs of owners of a row with the same first pivot
   std::unique_ptr<ChainGroups> groups;
   bool no_groups = false;         // no memory for them: the CTA kernel runs instead

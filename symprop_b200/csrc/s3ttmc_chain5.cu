@@ -63,8 +63,9 @@
 //
 // The first call on a tensor also orders its owners (chain_data: two radix sorts)
 // and deals them to the warps (chain5_build); both are kept.  First call, ms, FP32,
-// before this kernel / now: 250 nodes, 10,000 tuples, R = 8 1.02 / 0.92; 20,000 nodes,
-// 2M tuples, R = 16 16.7 / 10.4; 200,000 nodes, 20M tuples 127 / 95.
+// before this kernel / now: 250 nodes, 10,000 tuples, R = 8 1.02 / 0.67; 10,000 nodes,
+// 200,000 tuples 8.6 / 1.7; 20,000 nodes, 2M tuples, R = 16 16.7 / 10.3; 200,000 nodes,
+// 20M tuples 127 / 95.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -619,17 +620,20 @@ std::unique_ptr<ChainGroups> chain5_build(const TensorState &t, const ChainData 
   const size_t n = items.size();
   auto g = std::make_unique<ChainGroups>();
   g->sub.assign(n, 0);
-  g->first.alloc(n * kFirst);
-  g->S.alloc(t.nown * 4);
-  g->c.alloc(t.nown);
-  if (!n) return g;
+  Places pl;
+  const size_t at_S = pl.add<uint32_t>(t.nown * 4), at_c = pl.add<double>(t.nown), at_f = pl.add<uint32_t>(n * kFirst);
   cudaStream_t st = 0;
+  g->store.alloc(pl.bytes, st);
+  g->S = reinterpret_cast<uint32_t *>(g->store.p + at_S);
+  g->c = reinterpret_cast<double *>(g->store.p + at_c);
+  g->first = reinterpret_cast<uint32_t *>(g->store.p + at_f);
+  if (!n) return g;
   PoolBuf tmp(n * (sizeof(Chunk) + sizeof(uint32_t)), st);
   Chunk *const d = tmp.as<Chunk>();
   uint32_t *const count = reinterpret_cast<uint32_t *>(d + n);
   SPB_CUDA(cudaMemcpyAsync(d, items.data(), n * sizeof(Chunk), cudaMemcpyHostToDevice, st));
-  sub_groups_kernel<<<(unsigned)n, 128, 0, st>>>(d, cd.flags.p, count, reinterpret_cast<const uint4 *>(cd.S.p),
-                                                 cd.c64.p, reinterpret_cast<uint4 *>(g->S.p), g->c.p, g->first.p);
+  sub_groups_kernel<<<(unsigned)n, 128, 0, st>>>(d, cd.flags, count, reinterpret_cast<const uint4 *>(cd.S),
+                                                 cd.c64, reinterpret_cast<uint4 *>(g->S), g->c, g->first);
   SPB_LAUNCH_CHECK();
   SPB_CUDA(cudaMemcpyAsync(g->sub.data(), count, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
   SPB_CUDA(cudaStreamSynchronize(st));
@@ -641,9 +645,9 @@ void chain5_launch(const TensorState &t, const ChainData &cd, const ItemSet &ite
   GroupParams p{};
   p.chunks = items.chunks;
   p.nchunks = items.nchunks;
-  p.first = cd.groups->first.p;
-  p.S = cd.groups->S.p;
-  p.c = cd.groups->c.p;
+  p.first = cd.groups->first;
+  p.S = cd.groups->S;
+  p.c = cd.groups->c;
   p.U = dU;
   p.R = R;
   p.m = (uint32_t)symsize(R, 4);

@@ -342,9 +342,9 @@ void chain8_launch(const TensorState &t, const ChainData &cd, const ItemSet &ite
                    void *dYpacked, int precision, cudaStream_t st) {
   Params p;
   p.chunks = items.chunks;
-  p.S = cd.S.p;
-  p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64.p : (const void *)cd.c32.p;
-  p.flags = cd.flags.p;
+  p.S = cd.S;
+  p.c = precision == SYMPROP_FP64 ? (const void *)cd.c64 : (const void *)cd.c32;
+  p.flags = cd.flags;
   p.U = dU;
   p.R = R;
   p.m3 = (uint32_t)symsize(R, 3);
