@@ -138,12 +138,14 @@ __global__ void scale_kernel(const unsigned long long *cmax, int n, int *s, int 
 // may pass p / 2 by 2: put back into 8 bits where p / 2 + 2 > 127.
 // MAG: the last plane takes |n| 2^-53 in 7 bits, rounded down, and nsq the sum of
 // the squares of the same in 15 bits, rounded up (integers: the decision that
-// rests on them is the same in every run).
+// rests on them is the same in every run); weight (or null): its sum over the columns
+// for every block of 128 rows.
 template <bool MAG>
 __global__ void __launch_bounds__(128) residue_kernel(const double *__restrict__ A, int rows, int cols, int lda,
                                                       int chunk, int kc, const int *__restrict__ s, int chunk0,
                                                       signed char *__restrict__ out,
-                                                      unsigned long long *__restrict__ nsq, const Odd odd) {
+                                                      unsigned long long *__restrict__ nsq,
+                                                      unsigned long long *__restrict__ weight, const Odd odd) {
   if (odd.too_many()) return;
   constexpr int kPlanes = kP + (MAG ? 1 : 0);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
@@ -207,8 +209,25 @@ __global__ void __launch_bounds__(128) residue_kernel(const double *__restrict__
     __shared__ unsigned long long part[4][32];
     part[warp][lane] = sum;
     __syncthreads();
-    if (warp == 0 && c < cols)
-      atomicAdd(&nsq[(size_t)ch * cols + c], part[0][lane] + part[1][lane] + part[2][lane] + part[3][lane]);
+    if (warp == 0) {
+      sum = part[0][lane] + part[1][lane] + part[2][lane] + part[3][lane];
+      if (c < cols) atomicAdd(&nsq[(size_t)ch * cols + c], sum);
+      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      if (lane == 0 && weight) atomicAdd(&weight[blockIdx.z * gridDim.y + blockIdx.y], sum);
+    }
+  }
+}
+
+// The `few` blocks of 128 rows with the largest weight, per chunk (blockIdx.x)
+__global__ void __launch_bounds__(512) pick_kernel(const unsigned long long *weight, int kblocks, int few, int *picked) {
+  __shared__ unsigned long long w[kMaxChunk / 128];
+  const unsigned long long *mine = weight + (size_t)blockIdx.x * kblocks;
+  for (int i = threadIdx.x; i < kblocks; i += 512) w[i] = mine[i];
+  __syncthreads();
+  for (int i = threadIdx.x; i < kblocks; i += 512) {
+    int r = 0;
+    for (int j = 0; j < kblocks; ++j) r += w[j] > w[i] || (w[j] == w[i] && j < i);
+    if (r < few) picked[(size_t)blockIdx.x * few + r] = i;
   }
 }
 
@@ -245,7 +264,8 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 
 struct I8Args {
   int cols, ntile, ntiles;    // tiles of 256 per side, upper tiles
-  int kblocks, kstep;         // 128-wide blocks of a chunk: how many, every kstep-th
+  int kblocks;                // 128-wide blocks of a chunk
+  const int *picked;          // null: all of them, else kblocks of each chunk
   unsigned char *C;           // (chunk * kP + p) planes of ld x ld residues
   int ld;
   int *err;
@@ -318,6 +338,7 @@ __global__ void __launch_bounds__(256, 1)
   const uint32_t tmem = tmem_base_holder;
 
   if (warp == 0 && lane == 0) {
+    const int *picked = a.picked ? a.picked + (size_t)(plane / a.planes) * a.kblocks : nullptr;
     for (int it = 0; it < a.kblocks; ++it) {
       const int s = it % kNStages;
       const uint32_t round = (uint32_t)(it / kNStages);
@@ -327,8 +348,9 @@ __global__ void __launch_bounds__(256, 1)
       }
       unsigned char *st = smem + (size_t)s * 2 * kOperand;
       mbar_expect_tx(&full_bar[s], 2 * kOperand);
-      tma_load_2d(st, &map, &full_bar[s], it * a.kstep * kBK, row0);
-      tma_load_2d(st + kOperand, &map, &full_bar[s], it * a.kstep * kBK, col0);
+      const int x = (picked ? picked[it] : it) * kBK;
+      tma_load_2d(st, &map, &full_bar[s], x, row0);
+      tma_load_2d(st + kOperand, &map, &full_bar[s], x, col0);
       issued[s] = it + 1;
     }
   } else if (warp == 1 && lane == 0) {
@@ -510,15 +532,17 @@ int sms() {
 // most `limit` bytes, the one whose waves take least.  `nchunk` is 0 when there is
 // none.
 // The check of a componentwise Gram is a 17th plane among the sums, or (some rows give
-// a lower bound of W as well) two launches before them: every kstep-th block of 128 rows,
-// and all rows only where that is not enough.  The second costs two launches, the
-// first often a wave: 200,000 x 3,876 29.9 / 28.6 ms (without a check 27.4), 20,000 x
-// 2,002 1.15 / 1.09 (1.03); 20,000 x 320 0.315 / 0.333, 1,536 x 715 0.150 / 0.182.
+// a lower bound of W as well) launches before them: the eighth of the blocks of 128
+// rows that holds the largest rows, and all only where that is not enough.  The second
+// costs three launches, the first often a wave: 20,000 x 2,002 1.15 / 1.09 ms (without a
+// check 1.03); 20,000 x 320 0.315 / 0.333, 1,536 x 715 0.150 / 0.182.  Largest rows:
+// on rows with scales of a power law every 8th block left entries in doubt
+// (200,000 x 3,876: 29.6 ms).
 struct I8Plan {
   int ntile, ntiles, ld;
   int chunk, nchunk = 0;    // rows per chunk
   int kc, group;            // padded rows, chunks per launch
-  int kstep = 1;            // above 1: the check by itself, over every kstep-th block of rows first
+  int few = 0;              // not 0: the check by itself, over so many blocks of 128 rows first
   size_t res, bytes;        // of a launch's residues, and of all its operands
 };
 
@@ -544,26 +568,25 @@ I8Plan plan_i8(int rows, int cols, int planes, size_t limit) {
     const int kc = ((rows + c - 1) / c + kBK - 1) / kBK * kBK;
     int group = c;
     while (group > 1 && bytes(kc, group) > limit) --group;
-    // with the check among the sums' units, or (kstep > 1) before them
-    auto clocks = [&](int kstep) {
+    // with the check among the sums' units (few = 0), or before them
+    auto clocks = [&](int few) {
       double t = c * std::max(35000.0, 0.035 * cols * cols);
       auto launch = [&](double units, int kblocks) { t += std::ceil(units / n) * (kblocks * 1024.0 + 12000.0); };
       for (int x = 0; x < c; x += group) {
         const double part = (double)g.ntiles * std::min(group, c - x);
-        launch(part * (kstep > 1 ? kP : planes), kc / kBK);
-        if (kstep > 1) launch(part, kc / kBK / kstep), t += 50000.0;
+        launch(part * (few ? kP : planes), kc / kBK);
+        if (few) launch(part, few), t += 60000.0;
       }
       return t;
     };
-    const int some = planes > kP ? std::max(1, std::min(8, kc / kBK / 8)) : 1;
-    for (int kstep : {1, some}) {
-      const double t = clocks(kstep);
+    for (int few : {0, planes > kP ? kc / kBK / 8 : 0}) {
+      const double t = clocks(few);
       if (t < best) {
         best = t;
         g.nchunk = (rows + kc - 1) / kc;
         g.kc = kc;
         g.group = group;
-        g.kstep = kstep;
+        g.few = few;
       }
     }
   }
@@ -646,13 +669,18 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
   const Odd odd{list.as<int2>(), (unsigned *)(bad + 2), max_pairs(cols)};
   int *const suspect = bad + 3;
   if (componentwise) SPB_CUDA(cudaMemsetAsync(nsq.p, 0, ncs * 8, st));
+  const size_t nblocks = g.few ? (size_t)g.group * (g.kc / kBK) : 0;
+  PoolBuf blocks(nblocks * 8 + (size_t)g.group * g.few * sizeof(int), st);
+  unsigned long long *const weight = g.few ? blocks.as<unsigned long long>() : nullptr;
+  int *const picked = g.few ? reinterpret_cast<int *>(weight + nblocks) : nullptr;
   SPB_CUDA(cudaFuncSetAttribute(i8_gram_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
   for (int c0 = 0; c0 < g.nchunk; c0 += g.group) {
     const int nc = std::min(g.group, g.nchunk - c0);
+    if (g.few) SPB_CUDA(cudaMemsetAsync(weight, 0, nblocks * 8, st));
     auto residues = componentwise ? residue_kernel<true> : residue_kernel<false>;
     residues<<<dim3((cols + 31) / 32, g.kc / 128, nc), 128, 0, st>>>(A, rows, cols, lda, g.chunk, g.kc,
                                                                      (const int *)sc.p, c0, res,
-                                                                     (unsigned long long *)nsq.p, odd);
+                                                                     (unsigned long long *)nsq.p, weight, odd);
     SPB_LAUNCH_CHECK();
     CUtensorMap map;
     cuuint64_t dims[2] = {(cuuint64_t)g.kc, (cuuint64_t)nc * planes * cols};
@@ -677,18 +705,20 @@ bool gram_cols_i8(cudaStream_t st, const double *A, int rows, int cols, int lda,
     a.chunk = g.chunk;
     a.rows = rows;
     a.odd = odd;
-    auto product = [&](int checks, bool sums, int kstep = 1, bool some = false, int *suspect = nullptr) {
+    auto product = [&](int checks, bool sums, const int *picked = nullptr, int *suspect = nullptr) {
       a.checks = checks;
-      a.some = some;
+      a.some = picked != nullptr;
       a.suspect = suspect;
-      a.kstep = kstep;
-      a.kblocks = (g.kc / kBK + kstep - 1) / kstep;
+      a.picked = picked;
+      a.kblocks = picked ? g.few : g.kc / kBK;
       i8_gram_kernel<<<(unsigned)(g.ntiles * (checks + (sums ? nc * kP : 0))), 256, kSmem, st>>>(map, a);
       SPB_LAUNCH_CHECK();
     };
-    if (g.kstep > 1) {
-      product(nc, false, g.kstep, true, suspect);
-      product(nc, false, 1, false, suspect);
+    if (g.few) {
+      pick_kernel<<<nc, 512, 0, st>>>(weight, g.kc / kBK, g.few, picked);
+      SPB_LAUNCH_CHECK();
+      product(nc, false, picked, suspect);
+      product(nc, false, nullptr, suspect);
       product(0, true);
     } else {
       product(componentwise ? nc : 0, true);

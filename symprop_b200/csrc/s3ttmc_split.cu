@@ -61,6 +61,8 @@ constexpr int kTerms = 10;              // C(5, 3)
 constexpr int kMulWarps = 8, kMul = kMulWarps * 32;
 constexpr int kK = 16;                  // owners per stage
 constexpr int kStages = 2;
+// M of R = 11 has 36 x 9 tiles: 45 of a multiplying warp are 180 registers of sums
+// (it has 168), and in FP64 M and the panels are 268 KB of shared memory.
 constexpr int kMaxR = 10;
 
 // Sizes of the kernel for ranks up to RZ.  Panel rows are a multiple of 32

@@ -35,3 +35,21 @@ def test_integer_kernel_where_it_is_faster(gpu, n, m):
     G = gram(gpu, Y, gpu.FP64)
     assert column_errors(Y, G, [0, 255, 256, m // 2, m - 1]) <= 1.0
     assert diagonal_error(Y, G, np.arange(0, m, 7)) <= 4.0
+
+
+@pytest.mark.parametrize("odd", [False, True])
+def test_check_before_the_sums(gpu, odd):
+    """A width at which the check runs first, over the blocks with the largest rows: rows
+    with scales of a power law; columns whose large entry meets a zero, in a row of a
+    block that is not among them, go to the FP64 sums."""
+    import torch
+    n, m = 20011, 2002
+    Y = rows(n, m)
+    Y *= ((torch.randperm(n, generator=torch.Generator().manual_seed(1)) + 1).double() / n).pow(-0.45).cuda()[:, None]
+    if odd:
+        low = int(Y.abs().sum(1).view(-1)[: n // 128 * 128].view(-1, 128).sum(1).argmin()) * 128
+        Y[low + 3, 4], Y[low + 3, 5] = 1e17, 0.0
+        Y[n - 1, m - 1], Y[n - 1, 300] = 1e18, 0.0
+    G = gram(gpu, Y, gpu.FP64)
+    assert torch.equal(G, G.T)
+    assert column_errors(Y, G, [0, 4, 5, 300, m - 1]) <= 1.0
