@@ -168,8 +168,9 @@ int symprop_unpack_rows_device(const double *dpacked, uint64_t rows,
  * src/dense/matrixops.cpp:18-43; symsyrk :126-146 is its n x n twin).
  * precision SYMPROP_FP64: dY, dscale are double*; from 1,536 rows and 320
  * columns on integer tensor cores (exact sums of the columns rounded to 53
- * bits of their largest entry) where that keeps every entry within the rounding
- * bound of an FP64 sum, n 2^-53 sum_k |y_ki| |y_kj|, else FP64 CUDA-core GEMM;
+ * bits of their largest entry) where that is the faster way and keeps every entry
+ * within the rounding bound of an FP64 sum, n 2^-53 sum_k |y_ki| |y_kj|, else FP64
+ * CUDA-core GEMM;
  * SYMPROP_FP32: dY, dscale are float*, tcgen05 tensor cores with split-BF16
  * operands and FP32 accumulation. */
 int symprop_gram_device(const void *dY, uint64_t n, uint32_t m, const void *dscale,
@@ -354,11 +355,11 @@ int symprop_device_count(int *count);
 int symprop_set_device(int device);
 /* The library keeps the scratch of its dense steps (eigensolver blocks,
  * GEMM and Gram partial sums, the operands of the tensor-core Grams,
- * symsyrk_device and symgemm_device) in a per-device pool between calls, so that a
- * repeated solve allocates no new scratch: buffers of up to 4.5 GB, at most 9 GB in
+ * symsyrk_device and symgemm_device, a new tensor's sorts of up to 256 MB) in a
+ * per-device pool between calls, so that a repeated solve allocates no new scratch: buffers of up to 4.5 GB, at most 9 GB in
  * all; larger ones are given back when the call ends.  This waits for the current
- * device and returns the pool's unused memory to it (memory in use is not
- * touched); call it before handing the GPU to other work.  (No reference
+ * device and returns the pool's unused memory to it (memory in use, such as
+ * tensors' owners in pivot order of up to 64 MB, is not touched); call it before handing the GPU to other work.  (No reference
  * counterpart: the reference allocates host memory per call.) */
 int symprop_trim_memory(void);
 
